@@ -202,7 +202,10 @@ def executed_flops_per_traj_step(info, K):
     their non-zeros of the pruned pattern (2 live_nnz; the constant ones are
     a precomputed table), and per sub-step d Taylor terms of 2 flops per
     non-zero and 2 per row (its v term) plus one multiply per row (the
-    scaled form's 1/d!)."""
+    scaled form's 1/d!).  The power-series kernel multiplies by a constant
+    matrix: 2 per entry of it and 2 per row (the sum and its addition)."""
+    if info["variant"] == 8:
+        return K*(2*info["live_nnz"] + 2*info["rows"])
     nnz, rows, d, m = info["nnz"], info["rows"], info["degree"], info["substeps"]
     return K*(2*info["live_nnz"] + m*(d*(2*nnz + 2*rows) + rows))
 
@@ -216,7 +219,10 @@ def dense_flops_per_traj_step(N, G, K, m):
 def fp64_issue_per_traj_step(info, K, L):
     """FP64 warp instructions one trajectory step issues (its share of its
     group's instructions): d terms of fp64_per_term instructions per
-    exponential and sub-step, over the 32/L trajectories of a warp."""
+    exponential and sub-step, over the 32/L trajectories of a warp (the
+    power series has one term)."""
+    if info["variant"] == 8:
+        return K*info["fp64_per_term"]*L/32
     per_group = K*info["substeps"]*info["degree"]*info["fp64_per_term"]
     return per_group*min(L, 32)/32
 

@@ -307,7 +307,12 @@ int sss_plan_last_launches(const sss_plan* plan);
  * (sss_slot_layout), 8 to 256 lanes, up to 16 slots; 7 = phased row parts:
  * per lane C1 chains of P1 slots, a barrier, then C2 chains of P2 slots
  * that start from parked partial sums, every chain starting at a fixed
- * slot, 8, 16 or 32 lanes).  Automatic lanes: per lane count the cheapest
+ * slot, 8, 16 or 32 lanes; 8 = power series: an exponential as one
+ * multiplication by a constant sparse matrix on the powers of the varying
+ * coefficients, lab frame, at most two varying coefficients that are weak
+ * per step, up to 64 reachable rows, 16 to 128 lanes (above 32 a multiple
+ * of 32 up to the given count); automatic where it issues fewer FP64
+ * instructions than the Taylor action could).  Automatic lanes: per lane count the cheapest
  * layout (FP64 instructions per Horner term), and the lane count whose
  * busiest SM sub-partition issues the fewest of them.  Configured lanes
  * also set the adjoint's forward and backward groups; for sss_adjoint_run
@@ -357,11 +362,13 @@ int sss_slot_layout(int M, const int* row_ptr, const int* col, int lanes,
                     unsigned* words, int* entries);
 
 /* What the last batched run executes (no reference counterpart; for the
- * roofline count): the kernel variant chosen (1-7, as
+ * roofline count): the kernel variant chosen (1-8, as
  * sss_plan_set_batch_config), the generators assembled per exponential
  * (those whose coefficient varies; the constant ones are folded into a
  * table), their non-zeros on the pruned pattern, and the FP64 instructions
- * one group issues per Horner term.  Any pointer may be NULL. */
+ * one group issues per Horner term.  Variant 8: the varying coefficients,
+ * the entries of the series' matrices, and the FP64 instructions per
+ * exponential.  Any pointer may be NULL. */
 /* Shared-memory bank conflicts of the last slot-programmed layout (variants
  * 6 and 7; no reference counterpart): the extra wavefronts one Horner term
  * of one group costs, as modelled on the host from the layout's loads and

@@ -1192,7 +1192,7 @@ int adjoint_run(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg,
         return fail(SSS_EINVAL, "the differentiated channel must be a program channel with a "
                                 "generator (0 <= channel < nch, channel + 1 < G)");
     if (npar != 2 && npar != 4) return fail(SSS_EINVAL, "parameters per segment must be 2 or 4");
-    if (p->batch_variant == 0 || p->batch_variant == 4 || p->batch_variant == 5) {
+    if (p->batch_variant == 0 || p->batch_variant == 4 || p->batch_variant == 5 || p->batch_variant == 8) {
         const int rc = adjoint_run_parts(p, ntraj, d_rho0, nch, nseg, d_prog, t0, dt, T, F, h_rw,
                                          h_tw, dch, npar, d_J, d_grad, st);
         if (rc != SSS_EINVAL || p->batch_variant == 4 || p->batch_variant == 5) return rc;

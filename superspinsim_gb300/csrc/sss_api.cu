@@ -592,12 +592,12 @@ int sss_plan_set_batch_config(sss_plan* p, int lanes, int cta_threads, int varia
     if (!p) return fail(SSS_EINVAL, "null plan");
     if (lanes < 0 || lanes > 256 || (lanes & (lanes - 1)))
         return fail(SSS_EINVAL, "lanes must be 0 (automatic) or a power of two up to 256");
-    if (lanes > 32 && variant != 0 && variant != 4 && variant != 6)
-        return fail(SSS_EINVAL, "more than 32 lanes per trajectory needs the row-part or "
-                                "slot-packed variant");
+    if (lanes > 32 && variant != 0 && variant != 4 && variant != 6 && variant != 8)
+        return fail(SSS_EINVAL, "more than 32 lanes per trajectory needs the row-part, "
+                                "slot-packed or power-series variant");
     if (cta_threads != 0 && (cta_threads < 32 || cta_threads > 256 || cta_threads % 32))
         return fail(SSS_EINVAL, "cta_threads must be 0 or a multiple of 32 in [32, 256]");
-    if (variant < 0 || variant > 7) return fail(SSS_EINVAL, "variant must be 0 to 7");
+    if (variant < 0 || variant > 8) return fail(SSS_EINVAL, "variant must be 0 to 8");
     p->batch_lanes = lanes;
     p->batch_threads = cta_threads;
     p->batch_variant = variant;

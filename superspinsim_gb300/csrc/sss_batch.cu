@@ -1900,6 +1900,277 @@ int auto_lanes(const sss_plan* p, const double* cost, long n) {
     return auto_lane_count(4L * p->num_sms, cost, n);
 }
 
+int launch_power_l16(sss_plan* p, int E, int RM, const BatchArgs& a, int threads, size_t smem,
+                     cudaStream_t st);
+int launch_power_l32a(sss_plan* p, int E, int RM, const BatchArgs& a, int threads, size_t smem,
+                      cudaStream_t st);
+int launch_power_l32b(sss_plan* p, int E, int RM, const BatchArgs& a, int threads, size_t smem,
+                      cudaStream_t st);
+int launch_power_rows(sss_plan* p, int E, int W, const BatchArgs& a, int threads, size_t smem,
+                      cudaStream_t st);
+int launch_power_rows_cols(sss_plan* p, int E, int W, const BatchArgs& a, int threads, size_t smem,
+                           cudaStream_t st);
+int launch_power(sss_plan* p, int L, int E, int RM, const BatchArgs& a, int threads, size_t smem,
+                 cudaStream_t st) {
+    if (L > 32)
+        return a.cols ? launch_power_rows_cols(p, E, a.pw_w, a, threads, smem, st)
+                      : launch_power_rows(p, E, a.pw_w, a, threads, smem, st);
+    if (L == 16) return launch_power_l16(p, E, RM, a, threads, smem, st);
+    return E <= 14 ? launch_power_l32a(p, E, RM, a, threads, smem, st)
+                   : launch_power_l32b(p, E, RM, a, threads, smem, st);
+}
+
+// The power-series layout of a batch (sss_power.h) on the pruned pattern
+// row_ents: the series of every distinct constant part over the exponentials
+// of a step, packed for the lane count the automatic rule takes on its costs
+// (or the configured one).  horner_terms: the Taylor terms per exponential of
+// the other variants.  SSS_EINVAL when no layout fits or, unless `asked`, when
+// the Taylor action can do with fewer FP64 instructions: the series wins while
+// the varying coefficients are weak per step (one drive of the 7-level NV at
+// 5 ps: 27 instructions at 32 lanes against 8 x 5), and loses when two of them
+// are strong (the series in drive and laser of a Ramsey batch at 10 ps has
+// 1,264 entries against 9 x 106).
+static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vector<int>& active,
+                        const std::vector<double>& cmax, const std::vector<int>& rows_reached,
+                        const std::vector<std::vector<BatchLayout::Ent>>& row_ents, long nnz,
+                        int horner_terms, bool asked, BatchLayout* out) {
+    const int M = (int)rows_reached.size(), K = p->d.K, Q = p->d.Q, Ga = (int)active.size();
+    const SparseGenerators& sp = p->sparse;
+    BatchLayout& Ly = *out;
+    auto no = [](const char* why) {
+        return fail(SSS_EINVAL, std::string("power-series variant: ") + why);
+    };
+    if (p->rotating) return no("lab frame only");
+    if (p->d.taylor_degree > 0) return no("the plan fixes the Taylor degree");
+    if (M > kPowMaxRows) return no("too many reachable rows");
+    std::vector<int> live, fixed;   // active-generator indices
+    for (int gi = 0; gi < Ga; gi++) {
+        const int g = active[gi];
+        (Ly.slot_chan[g] >= 0 && !Ly.chan_const[g] ? live : fixed).push_back(gi);
+    }
+    if ((int)live.size() > kPowMaxLive) return no("too many varying coefficients");
+    std::vector<int> row_ptr(1, 0), col;
+    std::vector<int> ent_q;
+    for (const auto& re : row_ents) {
+        for (const BatchLayout::Ent& en : re) {
+            col.push_back(en.col);
+            ent_q.push_back(en.q);
+        }
+        row_ptr.push_back((int)col.size());
+    }
+    const double h = dt / F;
+    // the varying generators, scaled by the power of two that makes their
+    // coefficients at most 1
+    double wsum = 0.0;
+    for (int e = 0; e < K; e++) {
+        double s = 0.0;
+        for (int k = 0; k < Q; k++) s += std::fabs(p->W[e * Q + k]);
+        wsum = std::max(wsum, s);
+    }
+    std::vector<std::vector<double>> G(live.size());
+    std::vector<double> rho(live.size());
+    for (size_t i = 0; i < live.size(); i++) {
+        const int g = active[live[i]];
+        const double bound = cmax[g] * wsum * h;
+        if (!(bound > 0.0) || !std::isfinite(bound)) return no("unbounded coefficient");
+        int ex = 0;
+        rho[i] = std::frexp(bound, &ex);   // bound = rho 2^ex, rho < 1
+        if (ex < -900 || ex > 900) return no("coefficient out of range");
+        Ly.pw_scale[i] = std::ldexp(h, -ex);
+        for (int q : ent_q) G[i].push_back(std::ldexp(sp.val[(size_t)g * sp.nnz + q], ex));
+    }
+    // the constant part of each exponential, in double-double; equal ones
+    // (the two exponentials of CF4:2) share a table
+    using pow_detail::dd;
+    std::vector<std::vector<dd>> sums;   // per table: h sum_k W[e,k] X of each fixed generator
+    std::vector<std::vector<double>> A_hi, A_lo;
+    Ly.pw_tab.assign((size_t)K, 0);
+    for (int e = 0; e < K; e++) {
+        std::vector<dd> sv;
+        for (int gi : fixed) {
+            const int g = active[gi];
+            const double X = Ly.slot_chan[g] < 0 ? 1.0 : Ly.chan_value[g];
+            dd t{0.0, 0.0};
+            for (int k = 0; k < Q; k++)
+                t = pow_detail::dd_add(t, pow_detail::dd_mul({p->W[e * Q + k], 0.0}, {X, 0.0}));
+            sv.push_back(pow_detail::dd_mul(t, {h, 0.0}));
+        }
+        int at = -1;
+        for (size_t t = 0; t < sums.size() && at < 0; t++) {
+            bool same = true;
+            for (size_t i = 0; i < sv.size(); i++)
+                same = same && std::fabs((sums[t][i].hi - sv[i].hi) + (sums[t][i].lo - sv[i].lo)) <=
+                                   std::ldexp(std::fabs(sv[i].hi), -90);
+            if (same) at = (int)t;
+        }
+        if (at < 0) {
+            at = (int)sums.size();
+            sums.push_back(sv);
+            std::vector<double> hi(col.size()), lo(col.size());
+            for (size_t i = 0; i < col.size(); i++) {
+                dd a{0.0, 0.0};
+                for (size_t f = 0; f < fixed.size(); f++)
+                    a = pow_detail::dd_add(
+                        a, pow_detail::dd_mul(sv[f], {sp.val[(size_t)active[fixed[f]] * sp.nnz + ent_q[i]], 0.0}));
+                hi[i] = a.hi;
+                lo[i] = a.lo;
+            }
+            A_hi.push_back(hi);
+            A_lo.push_back(lo);
+        }
+        Ly.pw_tab[e] = at;
+    }
+    PowSeries ps;
+    if (!power_series(M, row_ptr, col, A_hi, A_lo, G, rho, &ps)) return no("the exponent is too large");
+    if (ps.ent.empty()) return no("nothing to do");
+    // lanes: the automatic rule on the costs of one exponential (two CTA
+    // barriers where a group is wider than a warp)
+    PowLayout lay[kLaneCounts];
+    double cost[kLaneCounts] = {}, chain[kLaneCounts] = {}, floor_cost[kLaneCounts] = {};
+    for (int i = 0; i < kLaneCounts; i++) {
+        const int L = 8 << i;
+        // no layout of the Taylor action issues less per exponential
+        // (at least four slots and, wider than a warp, two CTA barriers a term)
+        floor_cost[i] = (double)horner_terms * (std::max(4.0, (double)((nnz + M + L - 1) / L)) +
+                                                (L > 32 ? 1.0 : 0.0));
+        if (p->batch_lanes > 0 && p->batch_lanes != L) continue;
+        if (!power_pack(ps, L, &lay[i])) continue;
+        // issue figure (the CTA barrier and fewer groups to fill it cost a
+        // group wider than a warp about six instructions: 7-level sweep of
+        // 1024, 128 lanes 60 ms where their 13 instructions alone make 44)
+        // and chain, in units of the 66 cycles an instruction takes to issue
+        cost[i] = lay[i].cost() + (L > 32 ? 6.0 : 0.0);
+        chain[i] = lay[i].chain_cycles() / 66.0;
+    }
+    const long n = p->auto_lanes_ntraj > 0 ? p->auto_lanes_ntraj : ntraj;
+    const long sub = 4L * p->num_sms;
+    const int L = auto_lane_count(sub, cost, n, chain);
+    if (!L) return no("no layout fits");
+    int li = 0;
+    while ((8 << li) != L) li++;
+    if (!asked) {
+        // the Taylor action's terms: its issue, or its chain of about as many
+        // instructions and an exchange (3.5) per term
+        double fchain[kLaneCounts];
+        for (int i = 0; i < kLaneCounts; i++) fchain[i] = floor_cost[i] + 3.5 * horner_terms;
+        const int Lf = p->batch_lanes > 0 ? L : auto_lane_count(sub, floor_cost, n, fchain);
+        int fi = 0;
+        while ((8 << fi) != Lf) fi++;
+        if (lane_figure(sub, cost[li], n, L, chain[li]) > lane_figure(sub, floor_cost[fi], n, Lf, fchain[fi]))
+            return no("the Taylor action is cheaper");
+    }
+    for (int i = 0; i < kLaneCounts; i++) {
+        p->auto_cost[i] = cost[i];
+        p->auto_chain[i] = chain[i];
+    }
+    int threads = std::max(L, p->batch_threads > 0 ? std::min(p->batch_threads, 128) : 32);
+    if (L > 32) threads = lay[li].L;
+    if (L <= 32 && threads % L) return no("CTA size must be a multiple of the lanes per trajectory");
+    Ly.power = true;
+    Ly.ps = ps;
+    Ly.pl = lay[li];
+    Ly.pw_live = live;
+    Ly.L = lay[li].L;
+    Ly.E = lay[li].E;
+    Ly.S = lay[li].E;
+    Ly.npart = lay[li].n_part;
+    Ly.threads = threads;
+    Ly.degree = 0;
+    for (const auto& m : ps.mono) Ly.degree = std::max(Ly.degree, std::accumulate(m.begin(), m.end(), 0));
+    Ly.row_orig = rows_reached;
+    Ly.newpos.resize(M);
+    std::iota(Ly.newpos.begin(), Ly.newpos.end(), 0);
+    return SSS_OK;
+}
+
+// Kernel arguments and device tables of a power-series layout.
+static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int nseg, double dt,
+                           int F, const double* h_rw, DevBuf& tables, BatchArgs* out, size_t* smem,
+                           cudaStream_t st) {
+    const int M = Ly.M, L = Ly.L, E = Ly.E, Q = p->d.Q, K = p->d.K, N = p->d.N;
+    const PowSeries& ps = Ly.ps;
+    const PowLayout& pl = Ly.pl;
+    const int n_tab = ps.n_tables;
+    const size_t ne = ps.ent.size();
+    std::vector<double> dbl;
+    for (int t = 0; t < n_tab; t++)
+        for (int i = 0; i < E * L; i++)
+            dbl.push_back(pl.entry[i] >= 0 ? ps.val[t * ne + pl.entry[i]] : 0.0);
+    const size_t o_rw = dbl.size();
+    for (int k = 0; k < M; k++) dbl.push_back(h_rw ? h_rw[Ly.row_orig[k]] : 0.0);
+    const size_t o_toff = dbl.size();
+    for (int r = 0; r < F; r++) dbl.push_back(((double)r * dt) / F);
+    const size_t o_noff = dbl.size();
+    for (int k = 0; k < Q; k++) dbl.push_back((dt * p->nodes[k]) / F);
+    std::vector<int> ints(pl.xoff);
+    const size_t o_pb = ints.size();
+    ints.insert(ints.end(), pl.pbase.begin(), pl.pbase.end());
+    const size_t o_row = ints.size();
+    ints.insert(ints.end(), Ly.row_orig.begin(), Ly.row_orig.end());
+    const size_t o_help = ints.size();
+    ints.insert(ints.end(), pl.helper.begin(), pl.helper.end());
+    const size_t o_mask = ints.size();
+    for (unsigned w : pl.mask) ints.push_back((int)w);
+    const size_t o_merge = ints.size();
+    for (unsigned w : pl.merge) ints.push_back((int)w);
+    const size_t bytes = sizeof(double) * dbl.size() + sizeof(int) * ints.size();
+    if (int rc = tables.ensure(bytes + 64)) return rc;
+    std::vector<char> blob(bytes);
+    memcpy(blob.data(), dbl.data(), sizeof(double) * dbl.size());
+    memcpy(blob.data() + sizeof(double) * dbl.size(), ints.data(), sizeof(int) * ints.size());
+    SSS_CUDA(cudaMemcpyAsync(tables.p, blob.data(), bytes, cudaMemcpyHostToDevice, st));
+    if (int rc = p->w_queue.ensure(sizeof(int) * 4)) return rc;
+    SSS_CUDA(cudaMemsetAsync(p->w_queue.p, 0, sizeof(int) * 4, st));
+    const double* dv = tables.as<double>();
+    const int* di = reinterpret_cast<const int*>(dv + dbl.size());
+    BatchArgs a{};
+    a.M = M; a.Ga = Ly.Ga; a.K = K; a.Q = Q; a.F = F; a.nch = nch; a.nseg = nseg;
+    a.T_max = 0; a.ntraj = ntraj; a.degree = Ly.degree; a.substeps = 1; a.N = N;
+    a.E = E; a.S = E; a.npart = pl.n_part;
+    a.h_sub = dt / F; a.t0 = 0.0; a.dt = dt;
+    a.W = p->d_gens.as<double>() + p->gens.size();
+    a.pw_coef = dv;
+    a.rw = h_rw ? dv + o_rw : nullptr;
+    a.toff = dv + o_toff;
+    a.noff = dv + o_noff;
+    a.pw_x = di;
+    a.pcol = di + o_pb;
+    a.row_orig = di + o_row;
+    a.cw = reinterpret_cast<const unsigned*>(di + o_mask);
+    a.rbeg = di + o_help;
+    a.pw_merge = reinterpret_cast<const unsigned*>(di + o_merge);
+    a.pw_mono = (int)pl.mono.size();
+    a.pw_multi = n_tab > 1;
+    a.pw_w = pl.W;
+    a.kc = pl.copies;
+    for (int i = 0; i < a.pw_mono; i++) {
+        a.pw_p1[i] = (signed char)pl.p1[i];
+        a.pw_p2[i] = (signed char)pl.p2[i];
+    }
+    a.n_live = (int)Ly.pw_live.size();
+    a.n_lch = a.n_live;
+    for (int i = 0; i < a.n_live; i++) {
+        a.live_ch[i] = i;
+        a.lch_chan[i] = Ly.slot_chan[Ly.active[Ly.pw_live[i]]];
+        a.pw_scale[i] = Ly.pw_scale[i];
+    }
+    a.pw_sel_ch = -1;
+    for (int e = 0; e < K; e++)
+        for (int c = 0; c < (1 << kMaxQ); c++) a.pw_tab[(e << kMaxQ) + c] = (signed char)Ly.pw_tab[e];
+    a.tab_G = p->d.G;
+    a.queue = p->w_queue.as<int>();
+    p->mk_n_live = a.n_live;
+    p->mk_live_nnz = (int)ne;
+    p->last_bank_before = p->last_bank_after = 0;
+    *out = a;
+    const size_t ring = (size_t)(pl.rows ? kPowRowsRing : kRing);
+    const size_t per_slot = ((size_t)(pl.rows ? 2 * (a.pw_mono * M + 1) : M + 1 + pl.n_part + 1) +
+                             ring * (Q * a.n_lch + K * a.pw_mono) + a.pw_mono + ring * K / 2) | 1;
+    *smem = sizeof(double) * (pl.rows ? 1 : Ly.threads / L) * per_slot;
+    if (*smem > 227 * 1024) return fail(SSS_EINVAL, "power-series kernel: shared memory per CTA too large");
+    return SSS_OK;
+}
+
 int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg,
                  const double* d_prog, double dt, int F, const std::vector<int>& force_active,
                  bool allow_register, BatchLayout* out, cudaStream_t st, bool force_parts,
@@ -2066,6 +2337,20 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
     int degree, substeps;
     choose_taylor(beta, p->d.taylor_degree, &degree, &substeps);
 
+    // ---- power-series variant: automatic where it issues fewer FP64
+    // instructions than the Taylor action could, or asked for (8) ----
+    const bool power_asked = p->batch_variant == 8 && allow_register && !force_parts;
+    if (power_asked || (p->batch_variant == 0 && allow_register && !force_parts)) {
+        const int rc = power_layout(p, ntraj, dt, F, active, cmax, rows_reached, row_ents, nnz,
+                                    degree * substeps, power_asked, &Ly);
+        if (rc == SSS_OK) {
+            Ly.nnz = nnz;
+            Ly.substeps = 1;
+            return SSS_OK;
+        }
+        if (power_asked) return rc;
+    }
+
     // ---- lanes per trajectory ----
     // GB300 FP64 (~2 DFMA/clk/SM, 75-cycle latency) wants several warps per
     // SM.  Take the fewest lanes giving ~8 warps per SM, capped by the rows
@@ -2155,7 +2440,10 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
             chosen = L;
         } else {
             const long n_rule = p->auto_lanes_ntraj > 0 ? p->auto_lanes_ntraj : ntraj;
-            for (int i = 0; i < kLaneCounts; i++) p->auto_cost[i] = best_at(8 << i, false);
+            for (int i = 0; i < kLaneCounts; i++) {
+                p->auto_cost[i] = best_at(8 << i, false);
+                p->auto_chain[i] = 0.0;
+            }
             chosen = auto_lanes(p, p->auto_cost, n_rule);
         }
         if (chosen && best_at(chosen, true) > 0.0) {
@@ -2267,6 +2555,7 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
 static int make_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int nseg, double dt,
                      int F, const double* h_rw, const std::vector<int>& keep_live, DevBuf& tables,
                      BatchArgs* out, size_t* smem, cudaStream_t st) {
+    if (Ly.power) return make_power_args(p, Ly, ntraj, nch, nseg, dt, F, h_rw, tables, out, smem, st);
     const int M = Ly.M, Ga = Ly.Ga, L = Ly.L, E = Ly.E, degree = Ly.degree,
               substeps = Ly.substeps, threads = Ly.threads;
     const bool use_reg = Ly.use_reg;
@@ -2550,7 +2839,7 @@ int batch_prepare(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nse
     // samples, as a chunked run switches chunks.
     const bool phased = h_samples && ntraj > 1 && p->batch_lanes == 0 &&
                         (p->batch_variant == 0 || p->batch_variant == 4 || p->batch_variant == 5 ||
-                         p->batch_variant == 6 || p->batch_variant == 7);
+                         p->batch_variant == 6 || p->batch_variant == 7 || p->batch_variant == 8);
     if (phased) {
         p->batch_longest.assign(h_samples, h_samples + ntraj);
         std::sort(p->batch_longest.begin(), p->batch_longest.end(), std::greater<int>());
@@ -2588,6 +2877,8 @@ int batch_prepare(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nse
         ph.parts = Ly.parts;
         ph.slots = Ly.slots;
         ph.phased = Ly.phased;
+        ph.power = Ly.power;
+        ph.C = Ly.power ? Ly.pl.RM : ph.C;
         ph.S = Ly.S;
         ph.shape = Ly.shape;
         // the register-state form: one trajectory per warp, one chain per
@@ -2613,17 +2904,17 @@ int batch_prepare(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nse
             p->last_nnz = (int)Ly.nnz;
             p->last_epl = Ly.E;
             p->last_active = Ly.Ga;
-            p->last_variant = Ly.phased ? 7 : Ly.slots ? 6 : Ly.parts ? 4 : Ly.use_reg ? (ph.one_chain ? 3 : 1) : 2;
+            p->last_variant = Ly.power ? 8 : Ly.phased ? 7 : Ly.slots ? 6 : Ly.parts ? 4 : Ly.use_reg ? (ph.one_chain ? 3 : 1) : 2;
             p->last_n_live = p->mk_n_live;
             p->last_live_nnz = p->mk_live_nnz;
-            p->last_fp64_per_term = Ly.slots ? Ly.S : Ly.parts ? Ly.C * Ly.P + Ly.kc : Ly.E;
+            p->last_fp64_per_term = Ly.power ? Ly.pl.cost() : Ly.slots ? Ly.S : Ly.parts ? Ly.C * Ly.P + Ly.kc : Ly.E;
         }
-        if (!phased || !Ly.parts) break;
+        if (!phased || !(Ly.parts || Ly.power)) break;
         // the next phase starts at the first sample where the automatic
         // lane count for the trajectories still running exceeds this one
         // (phases only widen; where the count drops back to a narrower group
         // on a tie the phase runs on)
-        const int n_next = phase_end_count(4L * p->num_sms, p->auto_cost, Ly.L, running_after(p, t));
+        const int n_next = phase_end_count(4L * p->num_sms, p->auto_cost, Ly.L, running_after(p, t), p->auto_chain);
         if (n_next < 0 || p->batch_longest[n_next] <= t) break;
         t = p->batch_longest[n_next];
     }
@@ -2706,6 +2997,8 @@ int batch_launch(sss_plan* p, double* d_state, const double* d_prog, const int* 
         if (ph.shfl) {
             rc = ph.P == 4 ? launch(p, k_batch_shfl<4>, a, threads, threads / 32, smem, st)
                            : launch(p, k_batch_shfl<8>, a, threads, threads / 32, smem, st);
+        } else if (ph.power) {
+            rc = launch_power(p, L, ph.S, ph.C, a, threads, smem, st);
         } else if (ph.phased) {
             rc = launch_phased(p, L, ph.shape, a, threads, smem, st);
         } else if (ph.slots) {

@@ -77,6 +77,22 @@ struct BatchArgs {
     // final-state entry written so far is finite, else the smallest
     // (output sample << 32 | trajectory) that was not
     unsigned long long* health;
+    // power-series variant (sss_power.h): masks in cw, first partial sums in
+    // pcol, partial sums per trajectory in npart, the varying generators'
+    // channels in live_ch
+    const int* pw_x;           // E*L  offset of each slot's operand [q][l]
+    const double* pw_coef;     // tables*E*L  coefficients [table][q][l]
+    const unsigned* pw_merge;  // RM * M*pw_w  merge words [j][row*W + sub]
+    int pw_mono, pw_w, pw_multi;        // monomials, lanes per merged row, several tables
+    double pw_scale[kPowMaxLive];       // h times a power of two, per varying coefficient
+    signed char pw_p1[kPowMaxMono], pw_p2[kPowMaxMono];  // factors of each monomial value
+    signed char pw_tab[kMaxK << kMaxQ];  // table of (exponential, switched-channel code)
+    int pw_sel_ch;             // live-channel index of the switched channel, -1: none
+    double pw_sel_v;           // its second value (the code's set bits)
+    // propagator columns: a trajectory is column (index mod cols) of the
+    // propagators of a run of col_len samples, col_runs runs per trajectory
+    int cols, col_runs, col_len;
+    double* prop;              // [(trajectory*T_max + sample)*M + column]*M + row, identity subtracted
 };
 
 // Records a non-finite readout or final-state entry x of trajectory b at
@@ -164,6 +180,10 @@ int launch_slots_cta(sss_plan* p, int L, int S, const BatchArgs& a, int threads,
                      cudaStream_t st);
 int launch_phased(sss_plan* p, int L, int shape, const BatchArgs& a, int threads, size_t smem,
                   cudaStream_t st);
+// The power-series kernels for L lanes, E slots and RM merge slots
+// (sss_power_*.cu).
+int launch_power(sss_plan* p, int L, int E, int RM, const BatchArgs& a, int threads, size_t smem,
+                 cudaStream_t st);
 inline int launch_slots(sss_plan* p, int L, int S, const BatchArgs& a, int threads, size_t smem,
                         cudaStream_t st) {
     return L <= 32 ? launch_slots_warp(p, L, S, a, threads, smem, st)

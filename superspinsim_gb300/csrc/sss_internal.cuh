@@ -8,6 +8,7 @@
 
 #include "sss.h"
 #include "sss_lanes.h"
+#include "sss_power.h"
 
 namespace sss {
 
@@ -87,6 +88,15 @@ struct BatchLayout {
     std::vector<char> chan_const;            // per generator slot: its channel is batch-constant
     std::vector<double> chan_value;          // that constant
     std::vector<int> slot_chan;              // per generator slot: its program channel (-1: L0)
+    // power-series variant: the series, its program, the varying generators
+    // (active-generator indices), the power of two each coefficient is scaled
+    // by, and the table of every exponential
+    bool power = false;
+    PowSeries ps;
+    PowLayout pl;
+    std::vector<int> pw_live;
+    double pw_scale[kPowMaxLive] = {};
+    std::vector<int> pw_tab;
 };
 
 }  // namespace sss
@@ -139,17 +149,18 @@ struct sss_plan {
     bool ev_keep_begin = false;  // a later phase of one run: keep the first launch's begin event
     int auto_lanes_ntraj = 0;    // trajectories the automatic lane rule counts (0: the batch)
     double auto_cost[sss::kLaneCounts] = {};  // last automatic layout: cost per lane count 8..256
+    double auto_chain[sss::kLaneCounts] = {}; // and its chain figures (auto_lane_count)
     int launch_active = 0;       // trajectories with work in the next launch (0: the batch)
     // prepared batch (sss_batch_prepare -> sss_batch_launch): one kernel
     // layout per phase -- a single phase, or with uneven lengths and
     // automatic lanes one per widening lane count, phase k running from
     // output sample t_start on
     struct BatchPhase {
-        alignas(16) unsigned char args[1536];
+        alignas(16) unsigned char args[2048];
         size_t smem = 0;
         int L = 0, C = 0, P = 0, epl = 0, threads = 0, t_start = 0, S = 0, shape = 0;
         bool use_reg = false, one_chain = false, parts = false, shfl = false, slots = false,
-             phased = false;
+             phased = false, power = false;
     };
     BatchPhase batch_phase[sss::kMaxPhases];
     sss::DevBuf batch_tables[sss::kMaxPhases];
@@ -237,7 +248,7 @@ int parts_layout_rows(sss_plan* p, const std::vector<std::vector<BatchLayout::En
 // Row-part forward kernel prepared outside the plan's batch state (for the
 // adjoint): opaque kernel arguments and launch shape.
 struct PartsForward {
-    alignas(16) unsigned char args[1536];
+    alignas(16) unsigned char args[2048];
     size_t smem = 0;
     int L = 0, C = 0, P = 0, threads = 0;
 };

@@ -26,9 +26,17 @@ namespace sss {
 
 constexpr int kLaneCounts = 6;  // lanes per trajectory 8, 16, ..., 256 of the row kernels
 
+// the figure of one layout: the busiest sub-partition's issue, or the
+// dependent chain of a lone warp where that is longer (chain: in the same
+// units; 0: not counted)
+inline double lane_figure(long subparts, double cost, long n, long L, double chain) {
+    const long warps = (std::max(1L, n) * L + 31) / 32;
+    return std::max((double)((warps + subparts - 1) / subparts) * cost, chain);
+}
+
 // lanes per trajectory for n trajectories on `subparts` SM sub-partitions
-// (0: no lane count fits)
-inline int auto_lane_count(long subparts, const double* cost, long n) {
+// (0: no lane count fits); chain: the layouts' chains, or null
+inline int auto_lane_count(long subparts, const double* cost, long n, const double* chain = nullptr) {
     int best = 0;
     double best_v = 0.0;
     long best_warps = 0;
@@ -36,7 +44,7 @@ inline int auto_lane_count(long subparts, const double* cost, long n) {
         if (cost[i] <= 0.0) continue;
         const long Lc = 8L << i;
         const long warps = (std::max(1L, n) * Lc + 31) / 32;
-        const double v = (double)((warps + subparts - 1) / subparts) * cost[i];
+        const double v = lane_figure(subparts, cost[i], n, Lc, chain ? chain[i] : 0.0);
         if (!best || v < best_v || (v == best_v && best_warps < subparts)) {
             best = (int)Lc;
             best_v = v;
@@ -56,9 +64,10 @@ inline int running_after(const std::vector<int>& longest, int t) {
 // the running count, below n_now, at which a phase of L lanes ends: the
 // largest n < n_now for which the rule asks for more than L lanes (-1: the
 // phase runs to the end)
-inline int phase_end_count(long subparts, const double* cost, int L, int n_now) {
+inline int phase_end_count(long subparts, const double* cost, int L, int n_now,
+                           const double* chain = nullptr) {
     for (int n = n_now - 1; n >= 1; n--)
-        if (auto_lane_count(subparts, cost, n) > L) return n;
+        if (auto_lane_count(subparts, cost, n, chain) > L) return n;
     return -1;
 }
 

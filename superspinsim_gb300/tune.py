@@ -2,8 +2,8 @@
 
 Times short prepared launches of the actual batch (a few output samples of
 every trajectory) for each candidate configuration -- lanes per trajectory,
-kernel variant (two FMA chains per row, one, row parts, packed slots or
-phased row parts) and CTA size -- with CUDA events on the launch stream,
+kernel variant (two FMA chains per row, one, row parts, packed slots,
+phased row parts or the power series) and CTA size -- with CUDA events on the launch stream,
 keeps the fastest, and then, for that configuration, times a window of
 output samples run as launches of each candidate length (steps per launch,
 in output samples of F fine steps): short launches give finer resume
@@ -28,7 +28,7 @@ def _key(sweep, B, progs):
 
 
 def autotune(sweep, rho0, programs, time_step, samples=None, probe_samples=2, repeats=2,
-             lanes=(0, 8, 16, 32, 64, 128), variants=(1, 3, 4, 6, 7), threads=(32, 64, 128),
+             lanes=(0, 8, 16, 32, 64, 128), variants=(1, 3, 4, 6, 7, 8), threads=(32, 64, 128),
              chunks=(1, 4, 16, 64), chunk_tolerance=0.01, use_cache=True):
     """Pick and set the fastest batch configuration for this sweep and batch,
     then its launch length.  With uneven sample counts the lanes stay

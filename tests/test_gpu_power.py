@@ -1,0 +1,64 @@
+"""The power-series batched kernels (variant 8) against the oracle: every
+group width, one to nineteen reachable rows, none, one and two varying
+coefficients, one table (CF2:1, CF4:2) and several (CF6:5), uneven lengths
+and trajectories that outlast the coefficient ring."""
+import numpy as np
+import pytest
+
+from conftest import load_case, quadrature
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("lanes", [0, 16, 32, 64, 128])
+@pytest.mark.parametrize("name,K,drives", [("qubit_couple_res_e2", 2, 1), ("spin1_c1", 1, 1),
+                                           ("spin1_c1", 2, 0), ("spin1_c1", 2, 2),
+                                           ("spin1_c1", 5, 1), ("nv7_n19", 2, 1),
+                                           ("nv7_n49", 2, 2)])
+def test_power_series_against_oracle(name, K, drives, lanes):
+    from superspinsim_gb300 import _lib
+    c = load_case(name)
+    vm = c["vectorisation_map"]
+    gens = c["generators"]
+    N = vm.shape[0]
+    n = int(vm[:, 0].max()) + 1
+    rng = np.random.default_rng(17)
+    B, T, F, dt = 5, 5, 21, 1e-10
+    f0 = 28e6 if name.startswith("qubit") else 3.15e9
+    progs = np.zeros((B, 4, 2, 5))
+    progs[:, :, 0, 0] = 2.3e-10
+    progs[:, :, 1, 0] = np.inf
+    for ch in range(drives):
+        progs[:, ch, :, 1] = 1e-5*rng.uniform(-1, 1, (B, 2))
+        progs[:, ch, :, 2] = 1e-4*rng.uniform(0.2, 1, (B, 2))
+        progs[:, ch, :, 3] = f0*rng.uniform(0.9, 1.1, (B, 2))
+        progs[:, ch, :, 4] = rng.uniform(0, 6, (B, 2))
+    if n == 7:
+        progs[:, 3, :, 1] = 0.15
+    samples = np.array([T, 0, 1, T - 1, T], dtype=np.int32)
+    rho = np.zeros((n, n), complex)
+    rho[1, 1], rho[0, 0] = 0.75, 0.25
+    flat = np.stack([oracle.flatten(rho, vm, N)]*B)
+    w = rng.uniform(-1, 1, N)
+    W, nodes = quadrature(K)
+    plan = _lib.Plan(gens, W, nodes)
+    plan.set_batch_config(lanes=lanes, variant=8)
+    try:
+        ro, fin, tr = plan.batch(flat, progs, 0.0, dt, T, F, samples=samples, readout_weights=w,
+                                 want_final=True, want_trace=True)
+    except _lib.SSSError as e:
+        # more entries than this width's largest program holds
+        assert e.code == -1 and "no layout fits" in str(e)
+        assert lanes in (16, 32) or (n == 7 and drives == 2)
+        return
+    assert plan.batch_info()["variant"] == 8
+    _, ref = oracle.simulate(gens, np.stack([rho]*B), 0.0, T*dt + 1e-14, dt, progs, K=K, W=W,
+                             nodes=nodes, F=F, vectorisation_map=vm, mode="vector", degree=20,
+                             flat_out=True)
+    for b, s in enumerate(samples):
+        last = ref[b, s - 1] if s else flat[b]
+        assert np.abs(fin[b] - last).max() <= 1e-12
+        assert np.abs(tr[b, :s] - ref[b, :s]).max(initial=0.0) <= 1e-12
+        assert np.abs(ro[b, :s] - ref[b, :s] @ w).max(initial=0.0) <= 1e-12
+        assert not tr[b, s:].any() and not ro[b, s:].any()
