@@ -242,7 +242,13 @@ static int simulate_impl(sss_plan* p, int ntraj, const double* rho0, int nch, in
         }
         d_out = p->w_out.as<double>();
     }
-    int rc = plain_run(p, ntraj, d_rho0, nch, nseg, d_prog, d_tab, t0, dt, T, F, d_out, st);
+    // from host buffers by propagator columns where a layout fits, else (and
+    // from device buffers, whose call stays asynchronous) by dense propagators
+    int rc = host ? columns_run(p, ntraj, rho0, d_rho0, tab ? p->d.G : nch, tab ? 0 : nseg, tab ? nullptr : programs,
+                                tab ? nullptr : d_prog, d_tab, t0, dt, T, F, d_out, st)
+                  : SSS_EINVAL;
+    if (rc == SSS_EINVAL)
+        rc = plain_run(p, ntraj, d_rho0, nch, nseg, d_prog, d_tab, t0, dt, T, F, d_out, st);
     if (rc) return rc;
     if (host) {
         SSS_CUDA(cudaMemcpyAsync(out, d_out, sizeof(double) * (size_t)ntraj * T * N,
@@ -654,7 +660,8 @@ void sss_plan_destroy(sss_plan* p) {
                       &p->w_prop, &p->w_in, &p->w_out, &p->w_prog, &p->w_tab, &p->w_aux,
                       &p->w_queue, &p->w_ro, &p->w_fin, &p->w_samples, &p->w_status,
                       &p->w_state, &p->w_adjf, &p->w_adjb, &p->w_states, &p->w_adjro,
-                      &p->w_adjst, &p->w_order, &p->w_health};
+                      &p->w_adjst, &p->w_order, &p->w_health, &p->w_cols_tables,
+                      &p->w_cols_queue};
     for (DevBuf* b : bufs) b->release();
     for (DevBuf& b : p->batch_tables) b.release();
     if (p->ev_begin) cudaEventDestroy(p->ev_begin);

@@ -1297,7 +1297,7 @@ bool slots_try(const std::vector<int>& nent, const std::vector<int>& order, int 
 // first, then the barrier at S/2, each with the rows in decreasing size and
 // then in seeded random orders; the first layout that fits wins.
 bool slots_pack(const std::vector<int>& nent, int L, int S_cap, std::vector<SlotCell>& cell,
-                int* S_out, int* SA_out, int* npart_out) {
+                int* S_out, int* SA_out, int* npart_out, int max_tries = 4000) {
     const int M = (int)nent.size();
     long total = 0;
     for (int n : nent) total += n + 1;
@@ -1305,7 +1305,7 @@ bool slots_pack(const std::vector<int>& nent, int L, int S_cap, std::vector<Slot
     std::vector<int> base(M);
     std::iota(base.begin(), base.end(), 0);
     std::stable_sort(base.begin(), base.end(), [&](int x, int y) { return nent[x] > nent[y]; });
-    const int tries = std::max(8, std::min(4000, 60000 / std::max(1, M)));
+    const int tries = std::max(8, std::min(max_tries, 60000 / std::max(1, M)));
     for (int s = lo; s <= std::min(S_cap, kSlotsMax); s++) {
         if (!slot_size_compiled(s)) continue;
         for (int sa : {s, s / 2}) {
@@ -1735,7 +1735,7 @@ int slots_layout_rows(sss_plan* p, const std::vector<std::vector<BatchLayout::En
     for (int i = 0; i < M; i++) nent[i] = (int)rows[i].size();
     std::vector<SlotCell> cell;
     int S = 0, SA = 0, npart = 0;
-    if (!slots_pack(nent, L, S_cap, cell, &S, &SA, &npart))
+    if (!slots_pack(nent, L, S_cap, cell, &S, &SA, &npart, p->cols_samples ? 32 : 4000))
         return fail(SSS_EINVAL, "slot-packed variant does not fit this pattern at " + std::to_string(L) +
                                     " lanes per trajectory");
     if (int rc = emit_slot_cells(p, rows, cell, L, S, npart, active, rows_reached, Ly)) return rc;
@@ -1979,39 +1979,30 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
         Ly.pw_scale[i] = std::ldexp(h, -ex);
         for (int q : ent_q) G[i].push_back(std::ldexp(sp.val[(size_t)g * sp.nnz + q], ex));
     }
-    // the constant part of each exponential, in double-double; equal ones
-    // (the two exponentials of CF4:2) share a table
+    // the constant part of each exponential: the coefficients rounded as the
+    // Taylor kernels' (h sum_k W[e,k] X), their sum over the generators in
+    // double-double; equal ones (the two exponentials of CF4:2) share a table
     using pow_detail::dd;
-    std::vector<std::vector<dd>> sums;   // per table: h sum_k W[e,k] X of each fixed generator
-    std::vector<std::vector<double>> A_hi, A_lo;
+    std::vector<std::vector<double>> sums, A_hi, A_lo;
     Ly.pw_tab.assign((size_t)K, 0);
     for (int e = 0; e < K; e++) {
-        std::vector<dd> sv;
+        std::vector<double> sv;
         for (int gi : fixed) {
             const int g = active[gi];
             const double X = Ly.slot_chan[g] < 0 ? 1.0 : Ly.chan_value[g];
-            dd t{0.0, 0.0};
-            for (int k = 0; k < Q; k++)
-                t = pow_detail::dd_add(t, pow_detail::dd_mul({p->W[e * Q + k], 0.0}, {X, 0.0}));
-            sv.push_back(pow_detail::dd_mul(t, {h, 0.0}));
+            double t = 0.0;
+            for (int k = 0; k < Q; k++) t = std::fma(p->W[e * Q + k], X, t);
+            sv.push_back(t * h);
         }
-        int at = -1;
-        for (size_t t = 0; t < sums.size() && at < 0; t++) {
-            bool same = true;
-            for (size_t i = 0; i < sv.size(); i++)
-                same = same && std::fabs((sums[t][i].hi - sv[i].hi) + (sums[t][i].lo - sv[i].lo)) <=
-                                   std::ldexp(std::fabs(sv[i].hi), -90);
-            if (same) at = (int)t;
-        }
-        if (at < 0) {
-            at = (int)sums.size();
+        int at = (int)(std::find(sums.begin(), sums.end(), sv) - sums.begin());
+        if (at == (int)sums.size()) {
             sums.push_back(sv);
             std::vector<double> hi(col.size()), lo(col.size());
             for (size_t i = 0; i < col.size(); i++) {
                 dd a{0.0, 0.0};
                 for (size_t f = 0; f < fixed.size(); f++)
-                    a = pow_detail::dd_add(
-                        a, pow_detail::dd_mul(sv[f], {sp.val[(size_t)active[fixed[f]] * sp.nnz + ent_q[i]], 0.0}));
+                    a = pow_detail::dd_add(a, pow_detail::dd_mul({sv[f], 0.0},
+                                                                 {sp.val[(size_t)active[fixed[f]] * sp.nnz + ent_q[i]], 0.0}));
                 hi[i] = a.hi;
                 lo[i] = a.lo;
             }
@@ -2189,13 +2180,26 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
         nseg = 0;
     }
     auto slot_chan = [&](int a) { return rot ? a % p->d.G : (table ? a : a - 1); };
-    std::vector<double> h_rho0((size_t)ntraj * N), h_prog((size_t)ntraj * nch * nseg * 5);
-    SSS_CUDA(cudaMemcpyAsync(h_rho0.data(), d_rho0, sizeof(double) * h_rho0.size(),
-                             cudaMemcpyDeviceToHost, st));
-    if (!h_prog.empty())
-        SSS_CUDA(cudaMemcpyAsync(h_prog.data(), d_prog, sizeof(double) * h_prog.size(),
+    // the inputs on the host: the call's own buffers where it has them.  A
+    // projected plan's states are not in the generators' space: every row
+    // counts as reached
+    const bool all_rows = p->cols_samples && p->n_full;
+    const double *h_rho0 = p->host_rho0, *h_prog = p->host_prog;
+    std::vector<double> rho0_copy, prog_copy;
+    const size_t n_prog = (size_t)ntraj * nch * nseg * 5;
+    if (!h_rho0 && !all_rows) {
+        rho0_copy.resize((size_t)ntraj * N);
+        SSS_CUDA(cudaMemcpyAsync(rho0_copy.data(), d_rho0, sizeof(double) * rho0_copy.size(),
                                  cudaMemcpyDeviceToHost, st));
-    SSS_CUDA(cudaStreamSynchronize(st));
+        h_rho0 = rho0_copy.data();
+    }
+    if (!h_prog && n_prog) {
+        prog_copy.resize(n_prog);
+        SSS_CUDA(cudaMemcpyAsync(prog_copy.data(), d_prog, sizeof(double) * n_prog,
+                                 cudaMemcpyDeviceToHost, st));
+        h_prog = prog_copy.data();
+    }
+    if (!rho0_copy.empty() || !prog_copy.empty()) SSS_CUDA(cudaStreamSynchronize(st));
     // ---- channels: largest |coefficient|, and whether the channel holds one
     // constant value for every trajectory at all times (every segment of
     // zero amplitude with the same offset, the last one never ending; or
@@ -2254,7 +2258,8 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
     // largest), closed under the pattern and, rotating, the e^{L0 h} pairs ----
     std::vector<char> reach(N, 0);
     std::vector<int> stack;
-    for (int b = 0; b < ntraj; b++) {
+    if (all_rows) std::fill(reach.begin(), reach.end(), 1);
+    for (int b = 0; b < ntraj && !all_rows; b++) {
         const double* r0b = &h_rho0[(size_t)b * N];
         if (rot) {
             std::vector<double> xe(N, 0.0);
@@ -2295,6 +2300,14 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
     Ly.Ga = Ga;
     Ly.active = active;
     if (M == 0) return SSS_OK;
+    if (p->cols_samples) {
+        // as many columns as fill the SM sub-partitions with four warps of
+        // 8-lane groups each; fewer, longer runs past that (the states inside
+        // a run need no chain)
+        const long want = 16L * 4 * p->num_sms;
+        p->cols_len = (int)std::max(1L, (p->cols_samples * M + want - 1) / want);
+        p->auto_lanes_ntraj = (int)std::min(1L << 30, (p->cols_samples + p->cols_len - 1) / p->cols_len * M);
+    }
     if (M > 65534) return fail(SSS_EINVAL, "batched kernel supports at most 65534 reachable rows");
     std::vector<int> pos_of_orig(N, -1);
     for (int k = 0; k < M; k++) pos_of_orig[rows_reached[k]] = k;
@@ -2373,7 +2386,7 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
     const bool row_kernels = parts_asked || slots_asked || phased_asked;
     const bool slots_ok = !force_parts && (p->batch_variant == 0 || slots_asked);
     const bool phased_ok = !force_parts && (p->batch_variant == 0 || phased_asked);
-    const bool parts_ok = force_parts || (!slots_asked && !phased_asked);
+    const bool parts_ok = force_parts || (!slots_asked && !phased_asked && !p->cols_samples);
     if (rot && !force_parts && allow_register && p->batch_variant != 0 && !row_kernels)
         return fail(SSS_EINVAL, "the rotating frame runs on the row-part, slot-packed or phased "
                                 "kernel (variant 0, 4, 6 or 7)");
@@ -2447,7 +2460,8 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
             chosen = auto_lanes(p, p->auto_cost, n_rule);
         }
         if (chosen && best_at(chosen, true) > 0.0) {
-            rc = Ly.slots ? bank_relabel(p, Ly, active, varies) : SSS_OK;
+            // (a column run is too short to pay for the bank placement)
+            rc = Ly.slots && !p->cols_samples ? bank_relabel(p, Ly, active, varies) : SSS_OK;
         } else {
             const char* what = slots_asked ? "slot-packed" : phased_asked ? "phased row-part" : "row-part";
             rc = chosen ? fail(SSS_EINVAL, std::string(what) + " variant does not fit this pattern at " +
@@ -2746,6 +2760,7 @@ static int make_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int
             a.cfac[j] = c;
         }
         a.inv_dfact = 1.0 / a.cfac[1];
+        a.inv_dfact_lo = std::fma(-a.inv_dfact, a.cfac[1], 1.0) / a.cfac[1];
     }
     a.rot = rot ? 1 : 0;
     a.resid = (p->d.flags & SSS_RESIDUAL) ? 1 : 0;
@@ -2766,7 +2781,8 @@ static int make_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int
     *out = a;
     if (Ly.slots) {
         const size_t per_slot = (3 * (size_t)(M + 2 + Ly.npart) +
-                                 (size_t)kRing * (p->d.Q * lch.size() + p->d.K * live.size())) | 1;
+                                 (size_t)kRing * (p->d.Q * lch.size() + p->d.K * live.size()) +
+                                 (p->cols_samples ? (size_t)M : 0)) | 1;
         *smem = sizeof(double) * ((threads / L) * per_slot + M);
     } else if (Ly.parts) {
         const size_t per_slot = (3 * (size_t)(M + 2) + L * Ly.C + 1 +
@@ -2785,6 +2801,17 @@ static int make_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int
                                     " bytes of shared memory per CTA (max 232448); use fewer "
                                     "threads per CTA");
     return SSS_OK;
+}
+
+// Arguments and launch of a column run (sss_columns.cu).
+int batch_columns_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int nseg, double dt, int F,
+                       DevBuf& tables, BatchArgs* a, size_t* smem, cudaStream_t st) {
+    return make_args(p, Ly, ntraj, nch, nseg, dt, F, nullptr, {}, tables, a, smem, st);
+}
+int batch_columns_launch(sss_plan* p, const BatchLayout& Ly, const BatchArgs& a, size_t smem, cudaStream_t st) {
+    if (Ly.power) return launch_power(p, Ly.L, Ly.S, Ly.pl.RM, a, Ly.threads, smem, st);
+    if (Ly.phased) return launch_phased(p, Ly.L, Ly.shape, a, Ly.threads, smem, st);
+    return launch_slots(p, Ly.L, Ly.S, a, Ly.threads, smem, st);
 }
 
 // trajectories of a prepared batch with more than t output samples

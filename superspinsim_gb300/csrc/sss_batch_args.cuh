@@ -73,6 +73,7 @@ struct BatchArgs {
     unsigned amask[kMaxSlots]; // per live generator: slots with a non-zero value in some lane
     double cfac[kMaxTaylor + 1];  // scaled Horner: c_j = d!/(j-1)!
     double inv_dfact;          // 1/d!
+    double inv_dfact_lo;       // and the rounding error of that (propagator columns)
     // health word of the run, or null: all ones while every readout and
     // final-state entry written so far is finite, else the smallest
     // (output sample << 32 | trajectory) that was not
@@ -92,7 +93,8 @@ struct BatchArgs {
     // propagator columns: a trajectory is column (index mod cols) of the
     // propagators of a run of col_len samples, col_runs runs per trajectory
     int cols, col_runs, col_len;
-    double* prop;              // [(trajectory*T_max + sample)*M + column]*M + row, identity subtracted
+    double* prop;              // [(trajectory*(t_end - t_begin) + sample - t_begin)*M + column]*M + row,
+                               // the identity subtracted
 };
 
 // Records a non-finite readout or final-state entry x of trajectory b at
@@ -155,7 +157,7 @@ inline int launch(sss_plan* p, Kern kern, const BatchArgs& a, int threads, int s
     // captured into a graph (events recorded there cannot be waited on)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     SSS_CUDA(cudaStreamIsCapturing(st, &cap));
-    const bool timed = cap == cudaStreamCaptureStatusNone;
+    const bool timed = cap == cudaStreamCaptureStatusNone && !p->cols_samples;
     if (timed && !p->ev_begin) {
         SSS_CUDA(cudaEventCreate(&p->ev_begin));
         SSS_CUDA(cudaEventCreate(&p->ev_end));
@@ -167,7 +169,7 @@ inline int launch(sss_plan* p, Kern kern, const BatchArgs& a, int threads, int s
         SSS_CUDA(cudaEventRecord(p->ev_end, st));
         p->ev_recorded = true;
     }
-    p->last_grid = grid;
+    if (!p->cols_samples) p->last_grid = grid;
     return SSS_OK;
 }
 

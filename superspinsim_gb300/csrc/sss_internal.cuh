@@ -150,6 +150,15 @@ struct sss_plan {
     int auto_lanes_ntraj = 0;    // trajectories the automatic lane rule counts (0: the batch)
     double auto_cost[sss::kLaneCounts] = {};  // last automatic layout: cost per lane count 8..256
     double auto_chain[sss::kLaneCounts] = {}; // and its chain figures (auto_lane_count)
+    // a run by propagator columns being laid out or launched (sss_columns.cu):
+    // its samples over all trajectories (0: not one) and the samples per run;
+    // its launches record no timing events
+    long cols_samples = 0;
+    int cols_len = 1;
+    // the inputs of the call on the host, where it has them (null: the layout
+    // reads the device copies back)
+    const double *host_rho0 = nullptr, *host_prog = nullptr;
+    sss::DevBuf w_cols_tables, w_cols_queue;
     int launch_active = 0;       // trajectories with work in the next launch (0: the batch)
     // prepared batch (sss_batch_prepare -> sss_batch_launch): one kernel
     // layout per phase -- a single phase, or with uneven lengths and
@@ -193,6 +202,11 @@ namespace sss {
 int plain_run(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg,
               const double* d_prog, const double* d_tab, double t0, double dt,
               int T, int F, double* d_out, cudaStream_t st);
+// sss_columns.cu: the same by propagator columns on the batched kernels
+// (SSS_EINVAL: not for this plan, or no layout fits)
+int columns_run(sss_plan* p, int ntraj, const double* h_rho0, const double* d_rho0, int nch, int nseg,
+                const double* h_prog, const double* d_prog, const double* d_tab, double t0, double dt,
+                int T, int F, double* d_out, cudaStream_t st);
 // sss_batch.cu
 int batch_run(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg,
               const double* d_prog, const int* d_samples, const int* h_samples,

@@ -47,8 +47,8 @@ struct PowTrajectory {
             const int run = b / a.cols;
             col = b - run * a.cols;
             bt = run / a.col_runs;
-            t = (run - (int)bt * a.col_runs) * a.col_len;
-            T_b = min(t + a.col_len, a.T_max);
+            t = a.t_begin + (run - (int)bt * a.col_runs) * a.col_len;
+            T_b = min(t + a.col_len, a.t_end);
         } else {
             bt = b;
             T_b = min(a.samples ? a.samples[b] : a.T_max, a.t_end);
@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(128, 1) k_batch_power(const BatchArgs a) {
         if (++r == a.F) {
             r = 0;
             const int t = tr.t;
-            if (a.cols && keep) a.prop[((tr.bt * a.T_max + t) * (size_t)M + tr.col) * M + row] = acc;
+            if (a.cols && keep)
+                a.prop[((tr.bt * (a.t_end - a.t_begin) + t - a.t_begin) * (size_t)M + tr.col) * M + row] = acc;
             if (a.trace && keep) a.trace[((size_t)tr.b * a.T_max + t) * a.N + __ldg(a.row_orig + row)] = v;
             if (a.readout) {
                 double s = rw * v;
@@ -410,7 +411,8 @@ __global__ void __launch_bounds__(128, 1) k_batch_power_rows(const BatchArgs a) 
         if (++r == a.F) {
             r = 0;
             const int t = tr.t;
-            if (Cols && keep) a.prop[((tr.bt * a.T_max + t) * (size_t)M + tr.col) * M + row] = acc;
+            if (Cols && keep)
+                a.prop[((tr.bt * (a.t_end - a.t_begin) + t - a.t_begin) * (size_t)M + tr.col) * M + row] = acc;
             if (a.trace && keep) a.trace[((size_t)tr.b * a.T_max + t) * a.N + __ldg(a.row_orig + row)] = v;
             if (a.readout) {
                 double s = rw * v;

@@ -19,7 +19,7 @@
 // entries, because an entry's rounding is the same at every step: 2^-58 at
 // an entry of 0.05 would be a drift of 3e-12 over 800,000 exponentials.
 // Entries are dropped, smallest first, while the dropped sum of every
-// column stays below 2^-kPowDropBits.
+// column stays below a bound (kPowDrop).
 //
 // power_pack() deals the entries to the lanes of a group.
 #pragma once
@@ -34,10 +34,14 @@ namespace sss {
 constexpr int kPowMaxLive = 2;     // varying coefficients in the series
 constexpr int kPowMaxDegree = 8;   // total degree
 constexpr int kPowMaxMono = 24;    // monomial values per exponential (kernel ring)
-// entries and low parts below 2^-kPowDropBits of the state are dropped: 62
-// leaves the 16,000 exponentials of the 1024-frequency sweep at an error of
-// 3e-15, the Taylor action's; 58 drops 10 % more and drifts to 1.2e-13
-constexpr int kPowDropBits = 62;
+// Entries and low parts below 2^-62 of the state are dropped: the 16,000
+// exponentials of the 1024-frequency sweep keep the Taylor action's error of
+// 3e-15 (2^-58 drops 10 % more and drifts to 1.2e-13).  A propagator column is
+// kept minus its unit vector, so an exponent of norm x rounds it by 2^-53 x
+// only; over the 1/x exponentials that change it by its own size those
+// roundings add up to 2^-53 x^(1/2), a drop d to d/x: below x^(3/2) 2^-56 the
+// drop stays the smaller one.
+constexpr double kPowDrop = 0x1p-62, kPowDropSmall = 0x1p-56;
 constexpr int kPowMaxTables = 8;   // coefficient tables of a batch
 constexpr int kPowMaxRows = 64;    // reachable rows (the series fills in towards M^2)
 // FMA slots per lane and merge slots per row with a compiled kernel: groups of
@@ -224,7 +228,8 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
         }
     }
     // keep, per column, all but the smallest entries (by their largest value
-    // over the tables) whose sum stays below 2^-58
+    // over the tables) whose sum stays below the bound
+    const double drop = std::min(kPowDrop, kPowDropSmall * std::pow(x + b, 1.5));
     std::vector<char> keep((size_t)nm * MM, 0);
     std::vector<std::pair<double, size_t>> colv;
     std::vector<double> size(nm, 1.0);   // largest value of each monomial
@@ -244,7 +249,7 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
         double s = 0.0;
         for (const auto& e : colv) {
             s += e.first;
-            if (s > std::ldexp(1.0, -kPowDropBits)) keep[e.second] = 1;
+            if (s > drop) keep[e.second] = 1;
         }
     }
     ps.ent.clear();
@@ -256,7 +261,7 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
                 if (m == 0) {
                     double lo = 0.0;
                     for (int tab = 0; tab < n_tab; tab++) lo = std::max(lo, std::fabs(C0lo[tab][i]));
-                    if (lo > std::ldexp(1.0, -kPowDropBits)) {
+                    if (lo > drop) {
                         ps.ent.push_back({r, c, 0});
                         src.push_back({i, true});
                     }

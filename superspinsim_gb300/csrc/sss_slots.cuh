@@ -197,12 +197,14 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
     const int M = a.M, NL = a.n_live, NC = a.n_lch, K = a.K, Q = a.Q;
     const int Ms = M + 2 + a.npart;  // rows, zero row, sink row, partial sums
     const int slot = threadIdx.x / L, li = threadIdx.x % L;
-    const size_t per_slot = (3 * (size_t)Ms + (size_t)kRing * (Q * NC + K * NL)) | 1;
+    const size_t per_slot =
+        (3 * (size_t)Ms + (size_t)kRing * (Q * NC + K * NL) + (a.cols ? (size_t)M : 0)) | 1;
     double* V = smem + slot * per_slot;
     double* A = V + Ms;
     double* B = A + Ms;
     double* ringc = V + 3 * (size_t)Ms;          // [s][k][live channel] node values
     double* ring_ag = ringc + kRing * Q * NC;    // [s][e][live] CF weights
+    double* res = ring_ag + kRing * K * NL;      // propagator column minus its unit vector
     double* s_rw = smem + (size_t)(blockDim.x / L) * per_slot;
     for (int i = threadIdx.x; i < M; i += blockDim.x) s_rw[i] = a.rw ? a.rw[i] : 0.0;
     for (int i = li; i < 3 * Ms; i += L) V[i] = 0.0;
@@ -238,7 +240,8 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
     auto lds = [&](int off) { return *reinterpret_cast<const double*>(sb + off); };
     auto sts = [&](int off, double x) { *reinterpret_cast<double*>(sb + off) = x; };
     double om[S];
-    int b = -1, T_b = 0, t = 0, r = 0, rp = kRing;
+    int b = -1, T_b = 0, t = 0, r = 0, rp = kRing, col = -1;
+    size_t bt = 0;   // trajectory of the programs or the table
     const double* prog = nullptr;
     auto store_lab = [&](double* dst) {
         for (int i = li; i < a.N; i += L) {
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
 
     while (true) {
         if (r == 0 && t >= T_b) {
-            if (b >= 0 && a.fin) {
+            if (b >= 0 && a.fin && !a.cols) {
                 if (a.rot)
                     store_lab(a.fin + (size_t)b * a.N);
                 else
@@ -276,12 +279,26 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
             b = nb;
             if (b >= a.ntraj) break;
             if (a.order) b = __ldg(a.order + b);
+            bt = b;
             T_b = min(a.samples ? a.samples[b] : a.T_max, a.t_end);
             t = a.t_begin;
             rp = kRing;
-            prog = a.prog ? a.prog + (size_t)b * a.nch * a.nseg * 5 : nullptr;
+            if (a.cols) {
+                // column `col` of the propagators of a run of samples
+                const int run = b / a.cols;
+                col = b - run * a.cols;
+                bt = run / a.col_runs;
+                t = a.t_begin + (run - (int)bt * a.col_runs) * a.col_len;
+                T_b = min(t + a.col_len, a.t_end);
+            }
+            prog = a.prog ? a.prog + bt * a.nch * a.nseg * 5 : nullptr;
             const double* r0b = a.rho0 + (size_t)b * a.N;
-            if (a.rot) {
+            if (a.cols) {
+                for (int row = r0; row < r1; row++) {
+                    res[row] = 0.0;
+                    V[row] = row == col ? 1.0 : 0.0;
+                }
+            } else if (a.rot) {
                 for (int row = r0; row < r1; row++) {
                     const double* vi = a.Vinvm + (size_t)__ldg(a.row_orig + row) * a.N;
                     double o = 0.0;
@@ -302,7 +319,7 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
                 double val = 0.0;
                 if (a.tab) {
                     if (ts < a.T_max)
-                        val = __ldg(a.tab + (((size_t)b * a.F + rs) * a.T_max + ts) * (size_t)(Q * a.tab_G) +
+                        val = __ldg(a.tab + ((bt * a.F + rs) * a.T_max + ts) * (size_t)(Q * a.tab_G) +
                                     (size_t)k * a.tab_G + ch);
                 } else if (ch < a.nch) {
                     const double tn = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff + rs)),
@@ -361,8 +378,19 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
                 }
                 if (j == 1) program.template term<1>(om, 0.0, MsB, lds, sts, gsync);
                 // Omega u_1 is in A for odd d, B for even d
-                const double* res = (d & 1) ? A : B;
-                for (int row = r0; row < r1; row++) V[row] = fma(res[row], a.inv_dfact, V[row]);
+                const double* ou = (d & 1) ? A : B;
+                if (a.cols) {
+                    // (1/d! with its low part: the rounding of 1/d! alone is
+                    // the same at every exponential and would show in the
+                    // residual, 3e-16 after 5,000 of them on the qubit)
+                    for (int row = r0; row < r1; row++) {
+                        const double x = res[row] + fma(ou[row], a.inv_dfact, ou[row] * a.inv_dfact_lo);
+                        res[row] = x;
+                        V[row] = x + (row == col ? 1.0 : 0.0);
+                    }
+                } else {
+                    for (int row = r0; row < r1; row++) V[row] = fma(ou[row], a.inv_dfact, V[row]);
+                }
                 gsync();
             }
         }
@@ -372,15 +400,27 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
             for (int row = r0; row < r1; row++) {
                 const double xs = V[row], xp = V[__ldg(a.blk_pos + row)];
                 const double cs = __ldg(a.blk_self + row), cp = __ldg(a.blk_part + row);
-                A[row] = a.resid ? fma(cp, xp, fma(cs, xs, xs)) : fma(cp, xp, cs * xs);
+                if (a.cols) {
+                    const double unit = row == col ? 1.0 : 0.0;
+                    A[row] = a.resid ? fma(cp, xp, fma(cs, xs, res[row])) : fma(cp, xp, fma(cs, xs, -unit));
+                } else {
+                    A[row] = a.resid ? fma(cp, xp, fma(cs, xs, xs)) : fma(cp, xp, cs * xs);
+                }
             }
             gsync();
-            for (int row = r0; row < r1; row++) V[row] = A[row];
+            for (int row = r0; row < r1; row++) {
+                if (a.cols) res[row] = A[row];
+                V[row] = a.cols ? A[row] + (row == col ? 1.0 : 0.0) : A[row];
+            }
             gsync();
         }
         rp++;
         if (++r == a.F) {
             r = 0;
+            if (a.cols) {
+                double* dst = a.prop + ((bt * (a.t_end - a.t_begin) + t - a.t_begin) * (size_t)M + col) * M;
+                for (int row = r0; row < r1; row++) dst[row] = res[row];
+            }
             if (a.trace) {
                 if (a.rot)
                     store_lab(a.trace + ((size_t)b * a.T_max + t) * a.N);

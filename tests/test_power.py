@@ -4,7 +4,7 @@ program: on random sparse exponents the packed program of every lane count,
 run slot by slot as the kernels run it, gives e^{A + sum a G} x - x.  The
 reference is the Taylor action in long double.  Tolerance per row: the n
 products and sums of a row in binary64, n 2^-53 sum |c x| (doubled for the
-monomials' roundings), and the dropped entries, 2^-62 of every column.  No
+monomials' roundings), and the dropped entries, at most 2^-62 of every column.  No
 GPU."""
 import os
 import shutil
