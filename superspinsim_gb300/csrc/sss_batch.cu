@@ -1920,6 +1920,68 @@ int launch_power(sss_plan* p, int L, int E, int RM, const BatchArgs& a, int thre
                    : launch_power_l32b(p, E, RM, a, threads, smem, st);
 }
 
+// The constant samples of a batch (sss_constant.h): the sets of values its live
+// channels hold together and their maps, on the layout's reachable rows.
+static void constant_layout(sss_plan* p, BatchLayout& Ly, const double* h_prog, int ntraj, int nch, int nseg,
+                            double dt, int F) {
+    const int M = Ly.M, K = p->d.K, Q = p->d.Q;
+    const SparseGenerators& sp = p->sparse;
+    for (int g : Ly.active)
+        if (Ly.slot_chan[g] >= 0 && !Ly.chan_const[g]) Ly.cs_chan.push_back(Ly.slot_chan[g]);
+    if (Ly.cs_chan.empty()) return;
+    std::vector<int> row_ptr(1, 0), col, ent_q;
+    for (const auto& re : Ly.row_ents) {
+        for (const BatchLayout::Ent& en : re) {
+            col.push_back(en.col);
+            ent_q.push_back(en.q);
+        }
+        row_ptr.push_back((int)col.size());
+    }
+    using pow_detail::dd;
+    for (const ConstSet& set : constant_sets(h_prog, ntraj, nch, nseg, Ly.cs_chan, dt)) {
+        std::vector<std::vector<dd>> ex(K);
+        for (int e = 0; e < K; e++) {
+            ex[e].assign(col.size(), dd{0.0, 0.0});
+            for (int g : Ly.active) {
+                const int ch = Ly.slot_chan[g];
+                double X = ch < 0 ? 1.0 : Ly.chan_value[g], t = 0.0;
+                for (size_t i = 0; i < Ly.cs_chan.size(); i++)
+                    if (Ly.cs_chan[i] == ch) X = set.value[i];
+                for (int k = 0; k < Q; k++) t = std::fma(p->W[e * Q + k], X, t);
+                t *= dt / F;
+                for (size_t i = 0; i < col.size(); i++)
+                    ex[e][i] = pow_detail::dd_add(
+                        ex[e][i], pow_detail::dd_mul({t, 0.0}, {sp.val[(size_t)g * sp.nnz + ent_q[i]], 0.0}));
+            }
+        }
+        std::vector<double> hi, lo;
+        if (!constant_sample(M, F, row_ptr, col, ex, &hi, &lo)) continue;
+        Ly.cs.push_back(set);
+        for (const std::vector<double>* part : {&hi, &lo})
+            for (int c = 0; c < M; c++)
+                for (int r = 0; r < M; r++) Ly.cs_map.push_back((*part)[(size_t)r * M + c]);
+    }
+}
+
+// Appends a layout's constant-sample tables to the doubles of its device
+// blob: values per set in the order of the kernel's live channels, then the
+// maps with rows and columns in the layout's order.
+static void constant_tables(const BatchLayout& Ly, const std::vector<int>& lch, std::vector<double>& dbl,
+                            size_t* o_val, size_t* o_map) {
+    const int M = Ly.M, n = (int)Ly.cs.size();
+    *o_val = dbl.size();
+    for (const ConstSet& set : Ly.cs)
+        for (int ch : lch)
+            dbl.push_back(set.value[std::find(Ly.cs_chan.begin(), Ly.cs_chan.end(), ch) - Ly.cs_chan.begin()]);
+    *o_map = dbl.size();
+    dbl.resize(dbl.size() + (size_t)n * 2 * M * M);
+    for (int k = 0; k < 2 * n; k++)
+        for (int c = 0; c < M; c++)
+            for (int r = 0; r < M; r++)
+                dbl[*o_map + ((size_t)k * M + Ly.newpos[c]) * M + Ly.newpos[r]] =
+                    Ly.cs_map[((size_t)k * M + c) * M + r];
+}
+
 // The power-series layout of a batch (sss_power.h) on the pruned pattern
 // row_ents: the series of every distinct constant part over the exponentials
 // of a step, packed for the lane count the automatic rule takes on its costs
@@ -2093,6 +2155,10 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     for (int r = 0; r < F; r++) dbl.push_back(((double)r * dt) / F);
     const size_t o_noff = dbl.size();
     for (int k = 0; k < Q; k++) dbl.push_back((dt * p->nodes[k]) / F);
+    std::vector<int> lch;
+    for (int gi : Ly.pw_live) lch.push_back(Ly.slot_chan[Ly.active[gi]]);
+    size_t o_cval, o_cmap;
+    constant_tables(Ly, lch, dbl, &o_cval, &o_cmap);
     std::vector<int> ints(pl.xoff);
     const size_t o_pb = ints.size();
     ints.insert(ints.end(), pl.pbase.begin(), pl.pbase.end());
@@ -2140,9 +2206,12 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     }
     a.n_live = (int)Ly.pw_live.size();
     a.n_lch = a.n_live;
+    a.n_const = (int)Ly.cs.size();
+    a.cset = dv + o_cval;
+    a.cmat = dv + o_cmap;
     for (int i = 0; i < a.n_live; i++) {
         a.live_ch[i] = i;
-        a.lch_chan[i] = Ly.slot_chan[Ly.active[Ly.pw_live[i]]];
+        a.lch_chan[i] = lch[i];
         a.pw_scale[i] = Ly.pw_scale[i];
     }
     a.pw_sel_ch = -1;
@@ -2349,6 +2418,11 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
     beta *= wsum * dt / F;
     int degree, substeps;
     choose_taylor(beta, p->d.taylor_degree, &degree, &substeps);
+
+    // ---- samples over which nothing varies: one map per set of values ----
+    if (!table && !rot && allow_register && !force_parts && !p->cols_samples && M <= kConstMaxRows &&
+        F * p->d.K >= kConstMinExps)
+        constant_layout(p, Ly, h_prog, ntraj, nch, nseg, dt, F);
 
     // ---- power-series variant: automatic where it issues fewer FP64
     // instructions than the Taylor action could, or asked for (8) ----
@@ -2685,6 +2759,9 @@ static int make_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int
             ints.push_back(k);
         }
     }
+    size_t o_cval = 0, o_cmap = 0;
+    const bool constants = Ly.slots && keep_live.empty() && !Ly.cs.empty();
+    if (constants) constant_tables(Ly, lch, dbl, &o_cval, &o_cmap);
     size_t bytes = sizeof(double) * dbl.size() + sizeof(unsigned) * words.size() + sizeof(int) * ints.size();
     if (int rc = tables.ensure(bytes + 64)) return rc;
     std::vector<char> blob(bytes);
@@ -2739,6 +2816,11 @@ static int make_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int
             }
         p->mk_n_live = (int)live.size();
         p->mk_live_nnz = lnnz;
+    }
+    if (constants) {
+        a.n_const = (int)Ly.cs.size();
+        a.cset = dv + o_cval;
+        a.cmat = dv + o_cmap;
     }
     if (Ly.slots) {
         a.S = Ly.S;

@@ -90,6 +90,10 @@ struct BatchArgs {
     signed char pw_tab[kMaxK << kMaxQ];  // table of (exponential, switched-channel code)
     int pw_sel_ch;             // live-channel index of the switched channel, -1: none
     double pw_sel_v;           // its second value (the code's set bits)
+    // constant samples (sss_constant.h): sets, their values [set][live channel]
+    // and maps [set][hi, lo][column][row]
+    int n_const;
+    const double *cset, *cmat;
     // propagator columns: a trajectory is column (index mod cols) of the
     // propagators of a run of col_len samples, col_runs runs per trajectory
     int cols, col_runs, col_len;
@@ -103,6 +107,54 @@ struct BatchArgs {
 __device__ __forceinline__ void note_nonfinite(const BatchArgs& a, double x, int b, int t) {
     if (!isfinite(x) && a.health)
         atomicMin(a.health, ((unsigned long long)(unsigned)t << 32) | (unsigned)b);
+}
+
+// The set of constant values that the live channels hold over all of output
+// sample t, or -1: each in one segment of zero amplitude (or past its last)
+// from the first node of the sample to its last, at values of one of the
+// batch's sets.  Values no set holds (programs changed after the batch was
+// prepared) step as any others.
+__device__ __forceinline__ int constant_set(const BatchArgs& a, const double* prog, int t) {
+    if (!prog) return -1;
+    const double base = __dmul_rn(a.dt, (double)t);
+    const double t_first = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff)), base), __ldg(a.noff));
+    const double t_last = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff + a.F - 1)), base), __ldg(a.noff + a.Q - 1));
+    unsigned left = (1u << a.n_const) - 1u;
+    for (int ci = 0; ci < a.n_lch; ci++) {
+        const int ch = a.lch_chan[ci];
+        double val = 0.0;
+        if (ch < a.nch) {
+            const double* p = prog + (size_t)ch * a.nseg * 5;
+            for (int s = 0; s < a.nseg; s++, p += 5) {
+                if (!(t_first < p[0])) continue;
+                if (!(t_last < p[0]) || p[2] != 0.0) return -1;
+                val = p[1];
+                break;
+            }
+        }
+        for (int k = 0; k < a.n_const; k++)
+            if (__ldg(a.cset + k * a.n_lch + ci) != val) left &= ~(1u << k);
+    }
+    return __ffs((int)left) - 1;
+}
+
+// Row `row` of set k's map times the state v (M values), low parts first.
+__device__ __forceinline__ double constant_row(const BatchArgs& a, int k, const double* v, int row) {
+    const int M = a.M;
+    const double* p = a.cmat + (size_t)k * 2 * M * M + row;
+    double lo = 0.0, even = 0.0, odd = 0.0;
+    int c = 0;
+    for (; c + 1 < M; c += 2) {
+        lo = fma(__ldg(p + (size_t)(M + c) * M), v[c], lo);
+        even = fma(__ldg(p + (size_t)c * M), v[c], even);
+        lo = fma(__ldg(p + (size_t)(M + c + 1) * M), v[c + 1], lo);
+        odd = fma(__ldg(p + (size_t)(c + 1) * M), v[c + 1], odd);
+    }
+    if (c < M) {
+        lo = fma(__ldg(p + (size_t)(M + c) * M), v[c], lo);
+        even = fma(__ldg(p + (size_t)c * M), v[c], even);
+    }
+    return (even + odd) + lo;
 }
 
 // Slot words.

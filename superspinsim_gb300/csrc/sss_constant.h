@@ -1,0 +1,165 @@
+// Propagators of whole output samples over which nothing varies (host code,
+// used by sss_batch.cu; no reference counterpart).
+//
+// In a pulse protocol most samples are free evolution or plain laser: every
+// coefficient is constant from the sample's first node to its last, and the
+// F fine steps of K exponentials are the same linear map.  That map depends
+// only on the constant values, so a batch needs one matrix per set of values
+// -- laser on and laser off, for a Ramsey batch -- and a sample of it costs
+// one dense product in place of F K exponentials.  The matrices are formed in
+// double-double from the same rounded exponents as the kernels' and kept as
+// two doubles, minus the identity.
+#pragma once
+#include <algorithm>
+#include <cmath>
+#include <vector>
+
+#include "sss_power.h"
+
+namespace sss {
+
+constexpr int kConstMax = 8;       // sets of values of a batch
+constexpr int kConstMaxRows = 32;  // reachable rows (the products cost M^3 on the host)
+constexpr int kConstMinExps = 16;  // exponentials per sample a dense product is worth
+
+namespace pow_detail {
+
+using Matrix = std::vector<dd>;  // M x M row-major, a map minus the identity
+
+// (I + A)(I + B) - I
+inline Matrix compose(const Matrix& A, const Matrix& B, int M) {
+    Matrix C((size_t)M * M);
+    for (int r = 0; r < M; r++)
+        for (int c = 0; c < M; c++) {
+            dd s = dd_add(A[(size_t)r * M + c], B[(size_t)r * M + c]);
+            for (int k = 0; k < M; k++) {
+                const dd a = A[(size_t)r * M + k];
+                if (a.hi != 0.0) s = dd_add(s, dd_mul(a, B[(size_t)k * M + c]));
+            }
+            C[(size_t)r * M + c] = s;
+        }
+    return C;
+}
+
+// e^A - I by the Taylor series on the sparse pattern
+inline Matrix exponential(int M, const std::vector<int>& row_ptr, const std::vector<int>& col,
+                          const std::vector<dd>& A) {
+    Matrix T((size_t)M * M, dd{0.0, 0.0}), N(T), S(T);
+    for (int i = 0; i < M; i++) T[(size_t)i * M + i] = {1.0, 0.0};
+    for (int j = 1; j <= 60; j++) {
+        double big = 0.0;
+        for (int r = 0; r < M; r++) {
+            dd* n = &N[(size_t)r * M];
+            for (int c = 0; c < M; c++) n[c] = {0.0, 0.0};
+            for (int q = row_ptr[r]; q < row_ptr[r + 1]; q++) {
+                if (A[q].hi == 0.0) continue;
+                const dd* t = &T[(size_t)col[q] * M];
+                for (int c = 0; c < M; c++)
+                    if (t[c].hi != 0.0) n[c] = dd_add(n[c], dd_mul(A[q], t[c]));
+            }
+            for (int c = 0; c < M; c++) {
+                n[c] = dd_div(n[c], j);
+                S[(size_t)r * M + c] = dd_add(S[(size_t)r * M + c], n[c]);
+                big = std::max(big, std::fabs(n[c].hi));
+            }
+        }
+        T.swap(N);
+        if (big < 1e-36) break;
+    }
+    return S;
+}
+
+}  // namespace pow_detail
+
+// The map of F steps, each of the exponentials of `exponents` (the last acts
+// first), minus the identity: hi and lo parts, M x M row-major.  False when an
+// exponent's 1-norm exceeds 1 or is not finite.
+inline bool constant_sample(int M, int F, const std::vector<int>& row_ptr, const std::vector<int>& col,
+                            const std::vector<std::vector<pow_detail::dd>>& exponents,
+                            std::vector<double>* hi, std::vector<double>* lo) {
+    using namespace pow_detail;
+    const size_t MM = (size_t)M * M;
+    Matrix step(MM, dd{0.0, 0.0});
+    for (size_t e = 0; e < exponents.size(); e++) {
+        std::vector<double> s(M, 0.0);
+        for (size_t q = 0; q < col.size(); q++) s[col[q]] += std::fabs(exponents[e][q].hi);
+        for (double v : s)
+            if (!(v <= 1.0)) return false;
+        step = compose(step, exponential(M, row_ptr, col, exponents[e]), M);
+    }
+    Matrix out(MM, dd{0.0, 0.0});
+    bool any = false;
+    for (int n = F; n; n >>= 1) {
+        if (n & 1) {
+            out = any ? compose(out, step, M) : step;
+            any = true;
+        }
+        if (n > 1) step = compose(step, step, M);
+    }
+    hi->resize(MM);
+    lo->resize(MM);
+    for (size_t i = 0; i < MM; i++) {
+        (*hi)[i] = out[i].hi;
+        (*lo)[i] = out[i].lo;
+    }
+    return true;
+}
+
+// One set of values found constant together, and the time it lasts in all.
+struct ConstSet {
+    std::vector<double> value;   // per live channel
+    double total = 0.0;
+};
+
+// The sets of values that the live channels of a batch's programs
+// [b][channel][segment][5] hold together for at least dt, longest total first,
+// at most kConstMax.  A run's start and end are not known here: before the
+// first segment end and after the last one counts as long.
+inline std::vector<ConstSet> constant_sets(const double* prog, int ntraj, int nch, int nseg,
+                                           const std::vector<int>& live, double dt) {
+    std::vector<ConstSet> sets;
+    std::vector<double> cut;
+    for (int b = 0; b < ntraj; b++) {
+        cut.clear();
+        for (int ch : live)
+            for (int s = 0; s < nseg && ch < nch; s++) {
+                const double t = prog[(((size_t)b * nch + ch) * nseg + s) * 5];
+                if (std::isfinite(t)) cut.push_back(t);
+            }
+        std::sort(cut.begin(), cut.end());
+        for (size_t i = 0; i <= cut.size(); i++) {
+            const bool first = i == 0, last = i == cut.size();
+            const double from = first ? 0.0 : cut[i - 1], to = last ? 0.0 : cut[i];
+            const double length = first || last ? 1e3 * dt : to - from;
+            if (!(length >= dt)) continue;
+            const double at = first ? (last ? 0.0 : to - 0.5 * dt) : (last ? from + 0.5 * dt : 0.5 * (from + to));
+            std::vector<double> v;
+            for (int ch : live) {
+                double x = 0.0;
+                bool constant = true;
+                for (int s = 0; s < nseg && ch < nch; s++) {
+                    const double* sg = prog + (((size_t)b * nch + ch) * nseg + s) * 5;
+                    if (!(at < sg[0])) continue;
+                    constant = sg[2] == 0.0 && std::isfinite(sg[1]);
+                    x = sg[1];
+                    break;
+                }
+                if (!constant) break;
+                v.push_back(x);
+            }
+            if (v.size() != live.size()) continue;
+            size_t k = 0;
+            while (k < sets.size() && sets[k].value != v) k++;
+            if (k == sets.size()) {
+                if (sets.size() >= 64) continue;
+                sets.push_back({v, 0.0});
+            }
+            sets[k].total += length;
+        }
+    }
+    std::stable_sort(sets.begin(), sets.end(), [](const ConstSet& a, const ConstSet& b) { return a.total > b.total; });
+    if (sets.size() > (size_t)kConstMax) sets.resize(kConstMax);
+    return sets;
+}
+
+}  // namespace sss

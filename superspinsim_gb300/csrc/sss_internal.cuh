@@ -8,6 +8,7 @@
 
 #include "sss.h"
 #include "sss_lanes.h"
+#include "sss_constant.h"
 #include "sss_power.h"
 
 namespace sss {
@@ -97,6 +98,12 @@ struct BatchLayout {
     std::vector<int> pw_live;
     double pw_scale[kPowMaxLive] = {};
     std::vector<int> pw_tab;
+    // samples over which every live channel is constant (sss_constant.h): the
+    // live program channels, the sets of their values, and the maps minus the
+    // identity [set][hi, lo][column][row], rows in reachable order
+    std::vector<int> cs_chan;
+    std::vector<ConstSet> cs;
+    std::vector<double> cs_map;
 };
 
 }  // namespace sss

@@ -197,11 +197,22 @@ __global__ void __launch_bounds__(128, 1) k_batch_power(const BatchArgs a) {
             if (keep) X[row] = v;
             if (tr.t >= tr.T_b) continue;
         }
-        if (rp == R) {
+        const int cset = a.n_const && r == 0 ? constant_set(a, tr.prog, tr.t) : -1;
+        if (cset >= 0) {
+            // the whole sample by its map; the ring starts afresh after it
+            gsync();
+            const double d = own ? constant_row(a, cset, X, row) : 0.0;
+            gsync();
+            v += d;
+            if (keep) X[row] = v;
+            gsync();
+            rp = R;
+            r = a.F - 1;
+        } else if (rp == R) {
             pow_fill_ring<R>(a, tr, r, li, L, ringc, ring_m, ring_t, gsync);
             rp = 0;
         }
-        for (int i = 0; i < K; i++) {
+        for (int i = 0; i < K && cset < 0; i++) {
             const int re = rp * K + i;
             if (extra) {
                 const int tab = a.pw_multi ? ring_t[re] : 0;
@@ -266,7 +277,7 @@ __global__ void __launch_bounds__(128, 1) k_batch_power(const BatchArgs a) {
             if (keep) X[row] = v;
             gsync();
         }
-        rp++;
+        if (cset < 0) rp++;
         if (++r == a.F) {
             r = 0;
             const int t = tr.t;
@@ -364,13 +375,22 @@ __global__ void __launch_bounds__(128, 1) k_batch_power_rows(const BatchArgs a) 
                 v = a.rho0[(size_t)tr.b * a.N + __ldg(a.row_orig + row)];
             if (tr.t >= tr.T_b) continue;
         }
-        if (rp == R) {
+        const int cset = !Cols && a.n_const && r == 0 ? constant_set(a, tr.prog, tr.t) : -1;
+        if (cset >= 0) {
+            // the whole sample by its map; the ring starts afresh after it
+            if (keep) X[xb + row] = v;
+            gsync();
+            v += own ? constant_row(a, cset, X + xb, row) : 0.0;
+            gsync();
+            rp = R;
+            r = a.F - 1;
+        } else if (rp == R) {
             pow_fill_ring<R>(a, tr, r, li, L, ringc, ring_m, ring_t, gsync);
             rp = 0;
             write_x(0);
             gsync();
         }
-        for (int i = 0; i < K; i++) {
+        for (int i = 0; i < K && cset < 0; i++) {
             const int re = rp * K + i;
             if (extra) {
                 const int tab = a.pw_multi ? ring_t[re] : 0;
@@ -407,7 +427,7 @@ __global__ void __launch_bounds__(128, 1) k_batch_power_rows(const BatchArgs a) 
             write_x(re + 1);
             gsync();
         }
-        rp++;
+        if (cset < 0) rp++;
         if (++r == a.F) {
             r = 0;
             const int t = tr.t;

@@ -311,110 +311,121 @@ __global__ void __launch_bounds__(256, 1) k_batch_slots(const BatchArgs a) {
             gsync();
             if (t >= T_b) continue;
         }
-        if (rp == kRing) {
-            for (int i = li; i < kRing * Q * NC; i += L) {
-                const int s = i / (Q * NC), rem = i - s * Q * NC, k = rem / NC, ci = rem - k * NC;
-                const int rr = r + s, ts = t + rr / a.F, rs = rr % a.F;
-                const int ch = a.lch_chan[ci];
-                double val = 0.0;
-                if (a.tab) {
-                    if (ts < a.T_max)
-                        val = __ldg(a.tab + ((bt * a.F + rs) * a.T_max + ts) * (size_t)(Q * a.tab_G) +
-                                    (size_t)k * a.tab_G + ch);
-                } else if (ch < a.nch) {
-                    const double tn = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff + rs)),
-                                                          __dmul_rn(a.dt, (double)ts)),
-                                                __ldg(a.noff + k));
-                    val = channel_value(prog, a.nseg, ch, tn);
-                }
-                ringc[i] = val;
-            }
+        const int cset = a.n_const && r == 0 ? constant_set(a, prog, t) : -1;
+        if (cset >= 0) {
+            // the whole sample by its map; the ring starts afresh after it
+            for (int row = r0; row < r1; row++) A[row] = constant_row(a, cset, V, row);
             gsync();
-            for (int i = li; i < kRing * K * NL; i += L) {
-                const int s = i / (K * NL), rem = i - s * K * NL, e = rem / NL, gi = rem - e * NL;
-                const int kk = a.live_k[gi], ci = a.live_ch[gi];
-                double w = 0.0;
-                if (kk < 0) {
-                    for (int k = 0; k < Q; k++)
-                        w = fma(__ldg(a.W + e * Q + k), ringc[(s * Q + k) * NC + ci], w);
-                } else {
-                    w = __ldg(a.W + e * Q + kk) * ringc[(s * Q + kk) * NC + ci];
-                }
-                ring_ag[i] = w * a.h_sub;
-            }
+            for (int row = r0; row < r1; row++) V[row] += A[row];
             gsync();
-            rp = 0;
-        }
-        for (int e_exp = K - 1; e_exp >= 0; e_exp--) {
-            if (a.states) {
-                double* sp = a.states +
-                             (((size_t)b * a.st_steps + (size_t)(t - a.t_begin) * a.F + r) * K + e_exp) * M;
-                for (int row = r0; row < r1; row++) sp[row] = V[row];
-            }
-            const double* o0 = a.om0 + (size_t)e_exp * S * L + li;
-#pragma unroll
-            for (int q = 0; q < S; q++) om[q] = __ldg(o0 + (size_t)q * L);
-            for (int gi = 0; gi < NL; gi++) {
-                const double c = ring_ag[(rp * K + e_exp) * NL + gi];
-                if (is_zero(c)) continue;
-                const double* gv = a.gv + (size_t)a.live[gi] * S * L + li;
-                const unsigned am = a.amask[gi];
-#pragma unroll
-                for (int q = 0; q < S; q++)
-                    if ((am >> q) & 1u) om[q] = fma(c, __ldg(gv + (size_t)q * L), om[q]);
-            }
-            for (int m = 0; m < a.substeps; m++) {
-                // Horner terms j = d .. 1: V -> A, then A -> B, B -> A, ...
-                // The last term (j = 1) leaves the v term out and computes
-                // Omega u_1 alone; the row becomes v + (Omega u_1)/d!, so the
-                // rounded 1/d! scales only that small correction and no
-                // bias builds up in the state over many exponentials.
-                const int d = a.degree;
-                program.template term<0>(om, d == 1 ? 0.0 : a.cfac[d], 0, lds, sts, gsync);
-                int j = d - 1;
-                for (; j >= 2; j -= 2) {
-                    program.template term<1>(om, a.cfac[j], MsB, lds, sts, gsync);
-                    program.template term<2>(om, j == 2 ? 0.0 : a.cfac[j - 1], 0, lds, sts, gsync);
-                }
-                if (j == 1) program.template term<1>(om, 0.0, MsB, lds, sts, gsync);
-                // Omega u_1 is in A for odd d, B for even d
-                const double* ou = (d & 1) ? A : B;
-                if (a.cols) {
-                    // (1/d! with its low part: the rounding of 1/d! alone is
-                    // the same at every exponential and would show in the
-                    // residual, 3e-16 after 5,000 of them on the qubit)
-                    for (int row = r0; row < r1; row++) {
-                        const double x = res[row] + fma(ou[row], a.inv_dfact, ou[row] * a.inv_dfact_lo);
-                        res[row] = x;
-                        V[row] = x + (row == col ? 1.0 : 0.0);
+            rp = kRing;
+            r = a.F - 1;
+        } else {
+            if (rp == kRing) {
+                for (int i = li; i < kRing * Q * NC; i += L) {
+                    const int s = i / (Q * NC), rem = i - s * Q * NC, k = rem / NC, ci = rem - k * NC;
+                    const int rr = r + s, ts = t + rr / a.F, rs = rr % a.F;
+                    const int ch = a.lch_chan[ci];
+                    double val = 0.0;
+                    if (a.tab) {
+                        if (ts < a.T_max)
+                            val = __ldg(a.tab + ((bt * a.F + rs) * a.T_max + ts) * (size_t)(Q * a.tab_G) +
+                                        (size_t)k * a.tab_G + ch);
+                    } else if (ch < a.nch) {
+                        const double tn = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff + rs)),
+                                                              __dmul_rn(a.dt, (double)ts)),
+                                                    __ldg(a.noff + k));
+                        val = channel_value(prog, a.nseg, ch, tn);
                     }
-                } else {
-                    for (int row = r0; row < r1; row++) V[row] = fma(ou[row], a.inv_dfact, V[row]);
+                    ringc[i] = val;
+                }
+                gsync();
+                for (int i = li; i < kRing * K * NL; i += L) {
+                    const int s = i / (K * NL), rem = i - s * K * NL, e = rem / NL, gi = rem - e * NL;
+                    const int kk = a.live_k[gi], ci = a.live_ch[gi];
+                    double w = 0.0;
+                    if (kk < 0) {
+                        for (int k = 0; k < Q; k++)
+                            w = fma(__ldg(a.W + e * Q + k), ringc[(s * Q + k) * NC + ci], w);
+                    } else {
+                        w = __ldg(a.W + e * Q + kk) * ringc[(s * Q + kk) * NC + ci];
+                    }
+                    ring_ag[i] = w * a.h_sub;
+                }
+                gsync();
+                rp = 0;
+            }
+            for (int e_exp = K - 1; e_exp >= 0; e_exp--) {
+                if (a.states) {
+                    double* sp = a.states +
+                                 (((size_t)b * a.st_steps + (size_t)(t - a.t_begin) * a.F + r) * K + e_exp) * M;
+                    for (int row = r0; row < r1; row++) sp[row] = V[row];
+                }
+                const double* o0 = a.om0 + (size_t)e_exp * S * L + li;
+#pragma unroll
+                for (int q = 0; q < S; q++) om[q] = __ldg(o0 + (size_t)q * L);
+                for (int gi = 0; gi < NL; gi++) {
+                    const double c = ring_ag[(rp * K + e_exp) * NL + gi];
+                    if (is_zero(c)) continue;
+                    const double* gv = a.gv + (size_t)a.live[gi] * S * L + li;
+                    const unsigned am = a.amask[gi];
+#pragma unroll
+                    for (int q = 0; q < S; q++)
+                        if ((am >> q) & 1u) om[q] = fma(c, __ldg(gv + (size_t)q * L), om[q]);
+                }
+                for (int m = 0; m < a.substeps; m++) {
+                    // Horner terms j = d .. 1: V -> A, then A -> B, B -> A, ...
+                    // The last term (j = 1) leaves the v term out and computes
+                    // Omega u_1 alone; the row becomes v + (Omega u_1)/d!, so the
+                    // rounded 1/d! scales only that small correction and no
+                    // bias builds up in the state over many exponentials.
+                    const int d = a.degree;
+                    program.template term<0>(om, d == 1 ? 0.0 : a.cfac[d], 0, lds, sts, gsync);
+                    int j = d - 1;
+                    for (; j >= 2; j -= 2) {
+                        program.template term<1>(om, a.cfac[j], MsB, lds, sts, gsync);
+                        program.template term<2>(om, j == 2 ? 0.0 : a.cfac[j - 1], 0, lds, sts, gsync);
+                    }
+                    if (j == 1) program.template term<1>(om, 0.0, MsB, lds, sts, gsync);
+                    // Omega u_1 is in A for odd d, B for even d
+                    const double* ou = (d & 1) ? A : B;
+                    if (a.cols) {
+                        // (1/d! with its low part: the rounding of 1/d! alone is
+                        // the same at every exponential and would show in the
+                        // residual, 3e-16 after 5,000 of them on the qubit)
+                        for (int row = r0; row < r1; row++) {
+                            const double x = res[row] + fma(ou[row], a.inv_dfact, ou[row] * a.inv_dfact_lo);
+                            res[row] = x;
+                            V[row] = x + (row == col ? 1.0 : 0.0);
+                        }
+                    } else {
+                        for (int row = r0; row < r1; row++) V[row] = fma(ou[row], a.inv_dfact, V[row]);
+                    }
+                    gsync();
+                }
+            }
+            if (a.rot) {
+                // e^{L0 h} in the eigenbasis: each kept row from itself and its
+                // block partner, through A
+                for (int row = r0; row < r1; row++) {
+                    const double xs = V[row], xp = V[__ldg(a.blk_pos + row)];
+                    const double cs = __ldg(a.blk_self + row), cp = __ldg(a.blk_part + row);
+                    if (a.cols) {
+                        const double unit = row == col ? 1.0 : 0.0;
+                        A[row] = a.resid ? fma(cp, xp, fma(cs, xs, res[row])) : fma(cp, xp, fma(cs, xs, -unit));
+                    } else {
+                        A[row] = a.resid ? fma(cp, xp, fma(cs, xs, xs)) : fma(cp, xp, cs * xs);
+                    }
+                }
+                gsync();
+                for (int row = r0; row < r1; row++) {
+                    if (a.cols) res[row] = A[row];
+                    V[row] = a.cols ? A[row] + (row == col ? 1.0 : 0.0) : A[row];
                 }
                 gsync();
             }
+            rp++;
         }
-        if (a.rot) {
-            // e^{L0 h} in the eigenbasis: each kept row from itself and its
-            // block partner, through A
-            for (int row = r0; row < r1; row++) {
-                const double xs = V[row], xp = V[__ldg(a.blk_pos + row)];
-                const double cs = __ldg(a.blk_self + row), cp = __ldg(a.blk_part + row);
-                if (a.cols) {
-                    const double unit = row == col ? 1.0 : 0.0;
-                    A[row] = a.resid ? fma(cp, xp, fma(cs, xs, res[row])) : fma(cp, xp, fma(cs, xs, -unit));
-                } else {
-                    A[row] = a.resid ? fma(cp, xp, fma(cs, xs, xs)) : fma(cp, xp, cs * xs);
-                }
-            }
-            gsync();
-            for (int row = r0; row < r1; row++) {
-                if (a.cols) res[row] = A[row];
-                V[row] = a.cols ? A[row] + (row == col ? 1.0 : 0.0) : A[row];
-            }
-            gsync();
-        }
-        rp++;
         if (++r == a.F) {
             r = 0;
             if (a.cols) {
