@@ -122,8 +122,8 @@ __device__ __forceinline__ void park(unsigned addr, double x, unsigned yes) {
 template <int L, int E, int RM>
 __global__ void __launch_bounds__(128, 1) k_batch_power(const BatchArgs a) {
     extern __shared__ double smem[];
-    constexpr int NS = E >= 12 ? 2 : 1, S = E / NS, R = kRing;
-    static_assert(NS * S == E && L <= 32, "slots split evenly over the sequences");
+    constexpr int NS = E >= 12 ? 2 : 1, R = kRing;
+    static_assert(L <= 32, "a group lives in one warp");
     const int M = a.M, K = a.K, NM = a.pw_mono, W = a.pw_w;
     const int slot = threadIdx.x / L, li = threadIdx.x % L;
     const int n_x = M + 1, n_p = a.npart + 1;
@@ -237,15 +237,14 @@ __global__ void __launch_bounds__(128, 1) k_batch_power(const BatchArgs a) {
                     pp[i] = part_s + (unsigned)pb[i] * 8u;
                 }
 #pragma unroll
-                for (int q = 0; q < S; q++)
-#pragma unroll
-                    for (int i = 0; i < NS; i++) {
-                        const double base = ((start[i] >> q) & 1u) ? 0.0 : s[i];
-                        s[i] = fma(cf[i * S + q], x[i * S + q], base);
-                        const unsigned ends = (end[i] >> q) & 1u;
-                        park(pp[i], s[i], ends);
-                        pp[i] += ends * 8u;
-                    }
+                for (int q = 0; q < E; q++) {
+                    const int i = q % NS, k = q / NS;   // sequence, its slot
+                    const double base = ((start[i] >> k) & 1u) ? 0.0 : s[i];
+                    s[i] = fma(cf[q], x[q], base);
+                    const unsigned ends = (end[i] >> k) & 1u;
+                    park(pp[i], s[i], ends);
+                    pp[i] += ends * 8u;
+                }
             }
             gsync();
             const double* mv = ring_m + (size_t)re * NM;

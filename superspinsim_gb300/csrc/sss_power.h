@@ -46,7 +46,8 @@ constexpr int kPowMaxTables = 8;   // coefficient tables of a batch
 constexpr int kPowMaxRows = 64;    // reachable rows (the series fills in towards M^2)
 // FMA slots per lane and merge slots per row with a compiled kernel: groups of
 // 16 and of 32 lanes, and FMA slots of the row-aligned kernel (64 to 128)
-constexpr int kPowSlots[2][14] = {{8, 10, 12, 14, 16, 20, 24}, {2, 3, 4, 6, 8, 10, 12, 14, 16, 18, 20, 22, 24, 28}};
+constexpr int kPowSlots[2][16] = {{8, 10, 12, 14, 16, 20, 24},
+                                   {2, 3, 4, 6, 8, 10, 12, 14, 16, 17, 18, 19, 20, 22, 24, 28}};
 constexpr int kPowMerges[2][6] = {{3, 4, 5, 6, 8}, {3, 4, 5, 6, 7, 8}};
 constexpr int kPowRowSlots[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16, 20};
 template <int N>
@@ -283,7 +284,8 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
 // A group's program.
 //
 // 16 or 32 lanes (k_batch_power): L lanes of E slots, run as NS interleaved
-// sequences of E/NS slots (two from 12 slots on: two independent FMA chains).
+// sequences (two from 12 slots on, of ceil(E/2) and floor(E/2): two
+// independent FMA chains; slot q of sequence s is slot q NS + s of the lane).
 // The entries of a row that share a monomial form a list; the lists are laid
 // end to end over the sequences and cut where a sequence ends, so no slot is
 // padding until the last ones.  Every piece of a list is a partial sum; the
@@ -438,22 +440,26 @@ inline bool power_pack(const PowSeries& ps, int L, PowLayout* out) {
     if (!pow_monomials(ps, Ly, &at_mono)) return false;
     // lists: entries by row, then monomial (ps.ent is in that order already)
     Ly.NS = pow_sequences(Ly.E);
-    const int S = Ly.E / Ly.NS, seqs = L * Ly.NS;
+    const int seqs = L * Ly.NS;
+    auto length = [&](int sq) { return (Ly.E + Ly.NS - 1 - sq % Ly.NS) / Ly.NS; };
     Ly.entry.assign((size_t)Ly.E * L, -1);
     Ly.xoff.assign((size_t)Ly.E * L, M);
     Ly.mask.assign((size_t)Ly.NS * 2 * L, 0u);
     Ly.pbase.assign((size_t)Ly.NS * L, 0);
     std::vector<std::vector<unsigned>> merge(M);
-    // entries are spread evenly over the sequences, so the padding is too
-    int at = 0;
+    // entries are spread evenly over the sequences' slots, so the padding is
+    // too
+    int at = 0, before = 0;
     for (int sq = 0; sq < seqs; sq++) {
         const int l = sq / Ly.NS, s = sq % Ly.NS;
-        const int end = (int)((long)ne * (sq + 1) / seqs);
+        const int S = length(sq);
+        before += S;
+        const int end = (int)((long)ne * before / ((long)L * Ly.E));
         Ly.pbase[(size_t)s * L + l] = Ly.n_part;
         int q = 0, prow = -1, pm = -1;
         for (; at < end; at++, q++) {
             const PowEntry& e = ps.ent[at];
-            const size_t slot = (size_t)(s * S + q) * L + l;
+            const size_t slot = (size_t)(q * Ly.NS + s) * L + l;
             if (e.row != prow || e.mono != pm) {
                 if (prow >= 0) Ly.mask[(size_t)(2 * s + 1) * L + l] |= 1u << (q - 1);
                 Ly.mask[(size_t)(2 * s) * L + l] |= 1u << q;

@@ -42,6 +42,18 @@ int launch_power_l32b(sss_plan* p, int E, int RM, const BatchArgs& a, int thread
         SSS_POWER(32, 28, 6)
         SSS_POWER(32, 28, 7)
         SSS_POWER(32, 28, 8)
+        SSS_POWER(32, 17, 3)
+        SSS_POWER(32, 17, 4)
+        SSS_POWER(32, 17, 5)
+        SSS_POWER(32, 17, 6)
+        SSS_POWER(32, 17, 7)
+        SSS_POWER(32, 17, 8)
+        SSS_POWER(32, 19, 3)
+        SSS_POWER(32, 19, 4)
+        SSS_POWER(32, 19, 5)
+        SSS_POWER(32, 19, 6)
+        SSS_POWER(32, 19, 7)
+        SSS_POWER(32, 19, 8)
         default: return fail(SSS_EINVAL, "no power-series kernel for this layout");
     }
 }

@@ -63,14 +63,13 @@ static std::vector<double> run(const PowSeries& ps, const PowLayout& p, int tab,
     }
     std::vector<double> X(x), part(p.n_part + 1, 0.0);
     X.push_back(0.0);
-    const int S = p.E / p.NS;
     for (int l = 0; l < L; l++)
         for (int s = 0; s < p.NS; s++) {
             int pb = p.pbase[(size_t)s * L + l];
             double sum = 0.0;
-            for (int q = 0; q < S; q++) {
+            for (int q = 0; q * p.NS + s < p.E; q++) {
                 if ((p.mask[(size_t)(2 * s) * L + l] >> q) & 1u) sum = 0.0;
-                sum += coef(s * S + q, l) * X[p.xoff[(size_t)(s * S + q) * L + l]];
+                sum += coef(q * p.NS + s, l) * X[p.xoff[(size_t)(q * p.NS + s) * L + l]];
                 if ((p.mask[(size_t)(2 * s + 1) * L + l] >> q) & 1u) part[pb++] = sum;
             }
         }
