@@ -53,6 +53,8 @@
 
 namespace sss {
 
+constexpr int kLayoutMemos = 16;  // layout searches a plan remembers
+
 // ---------------------------------------------------------------------------
 // host: sparse pattern of the lab-frame generators
 // ---------------------------------------------------------------------------
@@ -63,6 +65,7 @@ int build_sparse(sss_plan* p) {
     // the basis change) are dropped
     const int N = p->d.N, G = p->rotating ? p->d.Q * p->d.G : p->d.G;
     SparseGenerators& s = p->sparse;
+    p->layout_memo.clear();  // layouts of other generators
     std::vector<double> drop(G, 0.0);
     if (p->rotating)
         for (int g = 0; g < G; g++) {
@@ -1292,6 +1295,66 @@ bool slots_try(const std::vector<int>& nent, const std::vector<int>& order, int 
     return true;
 }
 
+// Whether slots_try succeeds: its decisions without the cells.  The search
+// below fails thousands of orders for every one it keeps.
+struct SlotScratch {
+    std::vector<int> n, adds, donor, reserve;
+};
+bool slots_fits(const std::vector<int>& nent, const std::vector<int>& order, int L, int S, int SA,
+                SlotScratch& w) {
+    const bool bar = SA >= 1 && SA < S;
+    w.n.clear();
+    w.adds.clear();
+    w.donor.clear();
+    for (int i : order) {
+        const int n = nent[i];
+        int taken = 0, adds = 0;
+        if (n + 1 > S) {
+            if (!bar) return false;
+            while ((n - taken) + adds + 1 > S) {
+                const int k = std::min(SA, n - taken);
+                if (k <= 0) return false;
+                w.donor.push_back(k);
+                adds++;
+                taken += k;
+            }
+        }
+        w.n.push_back(n - taken);
+        w.adds.push_back(adds);
+    }
+    w.reserve.assign(L, 0);
+    int l = L - 1;
+    for (int k : w.donor) {
+        while (l >= 0 && w.reserve[l] + k > SA) l--;
+        if (l < 0) return false;
+        w.reserve[l] += k;
+    }
+    int lane = 0, pos = w.reserve[0];
+    for (size_t j = 0; j < w.n.size(); j++) {
+        const int m = w.adds[j], n = w.n[j] + m + 1;
+        while (true) {
+            if (lane >= L) return false;
+            if (pos + n <= S && (m == 0 || pos + w.n[j] >= SA)) {
+                pos += n;
+                if (pos == S) {
+                    lane++;
+                    pos = lane < L ? w.reserve[lane] : 0;
+                }
+                break;
+            }
+            const int recv_ents = S - pos - 1 - m, a = w.n[j] - recv_ents;
+            if (bar && recv_ents >= 0 && pos >= SA && a >= 1 && lane + 1 < L && w.reserve[lane + 1] + a <= SA) {
+                lane++;
+                pos = w.reserve[lane] + a;
+                break;
+            }
+            lane++;
+            pos = lane < L ? w.reserve[lane] : 0;
+        }
+    }
+    return true;
+}
+
 // Smallest compiled S (up to S_cap) with a slot layout of rows of nent
 // entries on L lanes: S from the lower bound ceil(sum(n+1)/L) up, with no cut
 // first, then the barrier at S/2, each with the rows in decreasing size and
@@ -1305,6 +1368,7 @@ bool slots_pack(const std::vector<int>& nent, int L, int S_cap, std::vector<Slot
     std::vector<int> base(M);
     std::iota(base.begin(), base.end(), 0);
     std::stable_sort(base.begin(), base.end(), [&](int x, int y) { return nent[x] > nent[y]; });
+    SlotScratch scratch;
     const int tries = std::max(8, std::min(max_tries, 60000 / std::max(1, M)));
     for (int s = lo; s <= std::min(S_cap, kSlotsMax); s++) {
         if (!slot_size_compiled(s)) continue;
@@ -1315,7 +1379,7 @@ bool slots_pack(const std::vector<int>& nent, int L, int S_cap, std::vector<Slot
             for (int t = 0; t < (sa == s ? 2 : tries); t++) {
                 if (t > 0) std::shuffle(ord.begin(), ord.end(), rng);
                 int np = 0;
-                if (slots_try(nent, ord, L, s, sa, cell, &np) && np < (1 << (32 - kSlotPidxShift))) {
+                if (slots_fits(nent, ord, L, s, sa, scratch) && slots_try(nent, ord, L, s, sa, cell, &np) && np < (1 << (32 - kSlotPidxShift))) {
                     *S_out = s;
                     *SA_out = sa;
                     *npart_out = np;
@@ -2231,6 +2295,28 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     return SSS_OK;
 }
 
+// What the row kernels' layout search depends on: the pattern (columns and
+// generator entries of every row), the active generators and which of them
+// vary, the rows' places in the state, and the configuration.
+static std::vector<int> layout_key(const std::vector<std::vector<BatchLayout::Ent>>& rows,
+                                   const std::vector<int>& active, const std::vector<int>& rows_reached,
+                                   const std::vector<char>& varies, std::initializer_list<int> config) {
+    std::vector<int> key(config);
+    for (const std::vector<int>* v : {&active, &rows_reached}) {
+        key.push_back((int)v->size());
+        key.insert(key.end(), v->begin(), v->end());
+    }
+    key.insert(key.end(), varies.begin(), varies.end());
+    for (const auto& re : rows) {
+        key.push_back((int)re.size());
+        for (const BatchLayout::Ent& en : re) {
+            key.push_back(en.col);
+            key.push_back(en.q);
+        }
+    }
+    return key;
+}
+
 int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg,
                  const double* d_prog, double dt, int F, const std::vector<int>& force_active,
                  bool allow_register, BatchLayout* out, cudaStream_t st, bool force_parts,
@@ -2521,21 +2607,43 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
             }
             return cost[pick];
         };
-        // lanes as configured, or the automatic count (auto_lanes)
+        // lanes as configured, or the automatic count (auto_lanes); the search
+        // is remembered in the plan (at most kLayoutMemos patterns)
         int rc = SSS_EINVAL, chosen = 0;
+        if (p->layout_memo.size() >= (size_t)kLayoutMemos) p->layout_memo.clear();
+        sss_plan::LayoutMemo& memo = p->layout_memo[layout_key(
+            Ly.row_ents, active, rows_reached, varies,
+            {threads_cfg, parts_ok, slots_ok, phased_ok, p->cols_samples > 0})];
         if (p->batch_lanes > 0) {
             chosen = L;
         } else {
             const long n_rule = p->auto_lanes_ntraj > 0 ? p->auto_lanes_ntraj : ntraj;
             for (int i = 0; i < kLaneCounts; i++) {
-                p->auto_cost[i] = best_at(8 << i, false);
+                if (!memo.costed) memo.cost[i] = best_at(8 << i, false);
+                p->auto_cost[i] = memo.cost[i];
                 p->auto_chain[i] = 0.0;
             }
+            memo.costed = true;
             chosen = auto_lanes(p, p->auto_cost, n_rule);
         }
-        if (chosen && best_at(chosen, true) > 0.0) {
+        const auto known = memo.built.find(chosen);
+        if (chosen && known != memo.built.end()) {
+            // the remembered layout with this batch's coefficients
+            BatchLayout t = known->second.layout;
+            t.chan_const = Ly.chan_const;
+            t.chan_value = Ly.chan_value;
+            t.slot_chan = Ly.slot_chan;
+            t.cs_chan = Ly.cs_chan;
+            t.cs = Ly.cs;
+            t.cs_map = Ly.cs_map;
+            Ly = t;
+            p->last_bank_before = known->second.bank_before;
+            p->last_bank_after = known->second.bank_after;
+            rc = SSS_OK;
+        } else if (chosen && best_at(chosen, true) > 0.0) {
             // (a column run is too short to pay for the bank placement)
             rc = Ly.slots && !p->cols_samples ? bank_relabel(p, Ly, active, varies) : SSS_OK;
+            if (rc == SSS_OK) memo.built[chosen] = {Ly, p->last_bank_before, p->last_bank_after};
         } else {
             const char* what = slots_asked ? "slot-packed" : phased_asked ? "phased row-part" : "row-part";
             rc = chosen ? fail(SSS_EINVAL, std::string(what) + " variant does not fit this pattern at " +

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <map>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -147,6 +148,21 @@ struct sss_plan {
     // generator values (the G^T block of the adjoint's block series)
     std::vector<double> slot_consts;
     std::unordered_map<uint64_t, std::vector<int>> bank_cache;
+    // row-kernel layouts found so far, by the pattern and configuration they
+    // depend on (layout_key in sss_batch.cu): the cost at every lane count and
+    // the layouts built, placed in their banks.  The search over lane counts
+    // and packings takes 13 to 95 ms of host time and depends on nothing else,
+    // so a sweep repeated on other programs of the same shape pays it once.
+    struct LayoutMemo {
+        double cost[sss::kLaneCounts] = {};
+        bool costed = false;
+        struct Built {
+            sss::BatchLayout layout;
+            int bank_before = 0, bank_after = 0;
+        };
+        std::map<int, Built> built;
+    };
+    std::map<std::vector<int>, LayoutMemo> layout_memo;
     int batch_variant = 0;  // 0: register variant when it fits, 2: shared-memory variant,
                             // 3: one-chain register variant, 4: row-part variant
     int device = 0;
