@@ -66,6 +66,7 @@ int build_sparse(sss_plan* p) {
     const int N = p->d.N, G = p->rotating ? p->d.Q * p->d.G : p->d.G;
     SparseGenerators& s = p->sparse;
     p->layout_memo.clear();  // layouts of other generators
+    p->series_memo.clear();
     std::vector<double> drop(G, 0.0);
     if (p->rotating)
         for (int g = 0; g < G; g++) {
@@ -1974,6 +1975,8 @@ int launch_power_rows(sss_plan* p, int E, int W, const BatchArgs& a, int threads
                       cudaStream_t st);
 int launch_power_rows_cols(sss_plan* p, int E, int W, const BatchArgs& a, int threads, size_t smem,
                            cudaStream_t st);
+int launch_power_big(sss_plan* p, int ctas, const BatchArgs& a, int threads, size_t smem, cudaStream_t st);
+int power_big_resident(int ctas);
 int launch_power(sss_plan* p, int L, int E, int RM, const BatchArgs& a, int threads, size_t smem,
                  cudaStream_t st) {
     if (L > 32)
@@ -2068,7 +2071,9 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
     };
     if (p->rotating) return no("lab frame only");
     if (p->d.taylor_degree > 0) return no("the plan fixes the Taylor degree");
-    if (M > kPowMaxRows) return no("too many reachable rows");
+    const bool big = M > kPowMaxRows;
+    if (M > kPowBigMaxRows || (big && (p->cols_samples || p->batch_lanes || p->batch_threads)))
+        return no("too many reachable rows");
     std::vector<int> live, fixed;   // active-generator indices
     for (int gi = 0; gi < Ga; gi++) {
         const int g = active[gi];
@@ -2116,9 +2121,10 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
         for (int gi : fixed) {
             const int g = active[gi];
             const double X = Ly.slot_chan[g] < 0 ? 1.0 : Ly.chan_value[g];
-            double t = 0.0;
-            for (int k = 0; k < Q; k++) t = std::fma(p->W[e * Q + k], X, t);
-            sv.push_back(t * h);
+            dd t{0.0, 0.0};   // rounded once, so that the order of the weights does not show
+            for (int k = 0; k < Q; k++)
+                t = pow_detail::dd_add(t, pow_detail::dd_mul({p->W[e * Q + k], 0.0}, {X, 0.0}));
+            sv.push_back(t.hi * h);
         }
         int at = (int)(std::find(sums.begin(), sums.end(), sv) - sums.begin());
         if (at == (int)sums.size()) {
@@ -2138,6 +2144,55 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
         Ly.pw_tab[e] = at;
     }
     PowSeries ps;
+    if (big) {
+        // one varying coefficient and one table: with two of either the
+        // tables outgrow shared memory
+        if (live.size() > 1 || A_hi.size() > 1) return no("a large system takes one varying coefficient and one table");
+        // the cluster that keeps every trajectory resident, and whether one
+        // could beat the Taylor action on a CTA per trajectory (measured on
+        // the 21-level NV: a term takes 105 cycles a slot and 500 at 128 lanes
+        // when each SM has one trajectory, and 64 a slot when it has more)
+        const long n = p->auto_lanes_ntraj > 0 ? p->auto_lanes_ntraj : ntraj;
+        int ctas = kPowBigMaxCtas;
+        while (ctas > 1 && n > power_big_resident(ctas)) ctas /= 2;
+        const double slots = (double)((nnz + M + 127) / 128), per_sm = std::ceil((double)n / p->num_sms);
+        const double taylor = horner_terms * std::max(105.0 * slots + 500.0, 64.0 * slots * per_sm);
+        std::vector<double> key{(double)M};
+        key.insert(key.end(), row_ptr.begin(), row_ptr.end());
+        key.insert(key.end(), col.begin(), col.end());
+        for (const auto* v : {&A_hi, &A_lo, &G})
+            for (const auto& x : *v) key.insert(key.end(), x.begin(), x.end());
+        key.insert(key.end(), rho.begin(), rho.end());
+        const auto hit = p->series_memo.find(key);
+        if (hit != p->series_memo.end()) {
+            ps = hit->second;
+        } else {
+            if (!power_series(M, row_ptr, col, A_hi, A_lo, G, rho, &ps)) return no("the exponent is too large");
+            if (p->series_memo.size() >= 8) p->series_memo.clear();
+            p->series_memo[key] = ps;
+        }
+        PowLayout pl;
+        if (!power_pack_big(ps, ctas, power_big_threads(ctas), &pl)) return no("no layout fits");
+        if (!asked && power_big_cycles(pl) * (ctas > 1 ? 1.0 : per_sm) > taylor)
+            return no("the Taylor action is cheaper");
+        for (int i = 0; i < kLaneCounts; i++) p->auto_cost[i] = p->auto_chain[i] = 0.0;
+        Ly.power = true;
+        Ly.ps = ps;
+        Ly.pl = pl;
+        Ly.pw_live = live;
+        Ly.L = Ly.threads = pl.L;
+        Ly.E = Ly.S = pl.E;
+        Ly.npart = 0;
+        Ly.degree = 0;
+        for (const auto& m : ps.mono) Ly.degree = std::max(Ly.degree, std::accumulate(m.begin(), m.end(), 0));
+        Ly.row_orig.resize(M);
+        Ly.newpos.resize(M);
+        for (int k = 0; k < M; k++) {
+            Ly.newpos[pl.order[k]] = k;
+            Ly.row_orig[k] = rows_reached[pl.order[k]];
+        }
+        return SSS_OK;
+    }
     if (!power_series(M, row_ptr, col, A_hi, A_lo, G, rho, &ps)) return no("the exponent is too large");
     if (ps.ent.empty()) return no("nothing to do");
     // lanes: the automatic rule on the costs of one exponential (two CTA
@@ -2211,8 +2266,7 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     const size_t ne = ps.ent.size();
     std::vector<double> dbl;
     for (int t = 0; t < n_tab; t++)
-        for (int i = 0; i < E * L; i++)
-            dbl.push_back(pl.entry[i] >= 0 ? ps.val[t * ne + pl.entry[i]] : 0.0);
+        for (int e : pl.entry) dbl.push_back(e >= 0 ? ps.val[t * ne + e] : 0.0);
     const size_t o_rw = dbl.size();
     for (int k = 0; k < M; k++) dbl.push_back(h_rw ? h_rw[Ly.row_orig[k]] : 0.0);
     const size_t o_toff = dbl.size();
@@ -2229,7 +2283,8 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     const size_t o_row = ints.size();
     ints.insert(ints.end(), Ly.row_orig.begin(), Ly.row_orig.end());
     const size_t o_help = ints.size();
-    ints.insert(ints.end(), pl.helper.begin(), pl.helper.end());
+    const std::vector<int>& rowsplit = pl.ctas ? pl.first_row : pl.helper;
+    ints.insert(ints.end(), rowsplit.begin(), rowsplit.end());
     const size_t o_mask = ints.size();
     for (unsigned w : pl.mask) ints.push_back((int)w);
     const size_t o_merge = ints.size();
@@ -2287,6 +2342,13 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     p->mk_live_nnz = (int)ne;
     p->last_bank_before = p->last_bank_after = 0;
     *out = a;
+    if (pl.ctas) {
+        *smem = sizeof(double) * (2 * (size_t)(a.pw_mono * M + 1) +
+                                  (size_t)pow_big_ring(pl.ctas) * (Q * a.n_lch + K * a.pw_mono) + a.pw_mono) +
+                (sizeof(double) + sizeof(unsigned short)) * (size_t)E * L;
+        if (*smem > 226 * 1024) return fail(SSS_EINVAL, "power-series kernel: shared memory per CTA too large");
+        return SSS_OK;
+    }
     const size_t ring = (size_t)(pl.rows ? kPowRowsRing : kRing);
     const size_t per_slot = ((size_t)(pl.rows ? 2 * (a.pw_mono * M + 1) : M + 1 + pl.n_part + 1) +
                              ring * (Q * a.n_lch + K * a.pw_mono) + a.pw_mono + ring * K / 2) | 1;
@@ -3096,6 +3158,7 @@ int batch_prepare(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nse
         ph.phased = Ly.phased;
         ph.power = Ly.power;
         ph.C = Ly.power ? Ly.pl.RM : ph.C;
+        ph.P = Ly.power ? Ly.pl.ctas : ph.P;
         ph.S = Ly.S;
         ph.shape = Ly.shape;
         // the register-state form: one trajectory per warp, one chain per
@@ -3214,6 +3277,8 @@ int batch_launch(sss_plan* p, double* d_state, const double* d_prog, const int* 
         if (ph.shfl) {
             rc = ph.P == 4 ? launch(p, k_batch_shfl<4>, a, threads, threads / 32, smem, st)
                            : launch(p, k_batch_shfl<8>, a, threads, threads / 32, smem, st);
+        } else if (ph.power && ph.P) {
+            rc = launch_power_big(p, ph.P, a, threads, smem, st);
         } else if (ph.power) {
             rc = launch_power(p, L, ph.S, ph.C, a, threads, smem, st);
         } else if (ph.phased) {

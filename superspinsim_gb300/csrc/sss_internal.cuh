@@ -163,6 +163,9 @@ struct sss_plan {
         std::map<int, Built> built;
     };
     std::map<std::vector<int>, LayoutMemo> layout_memo;
+    // power series of large systems by the matrices they were made from (25 ms
+    // of host time at 171 rows): pattern, constant parts, varying generators
+    std::map<std::vector<double>, sss::PowSeries> series_memo;
     int batch_variant = 0;  // 0: register variant when it fits, 2: shared-memory variant,
                             // 3: one-chain register variant, 4: row-part variant
     int device = 0;

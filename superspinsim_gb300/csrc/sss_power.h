@@ -304,6 +304,8 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
 struct PowLayout {
     int L = 0, E = 0, NS = 1, RM = 0, W = 1;
     bool rows = false;
+    int ctas = 0;                           // CTAs of a cluster (power_pack_big), 0: not one
+    std::vector<int> order, first_row;      // its rows in the layout's order, each CTA's together
     int copies = 1;                         // row-aligned: copies written per lane
     std::vector<std::vector<int>> mono;     // ring values: exponents of each monomial, by degree
     int p1[kPowMaxMono] = {}, p2[kPowMaxMono] = {};   // value i = value p1 * coefficient p2
@@ -322,7 +324,7 @@ struct PowLayout {
         return lg;
     }
     // FP64 instructions of one exponential
-    int cost() const { return rows ? E + log_w() + 1 + copies : E + RM + std::max(log_w(), 1) + 1; }
+    int cost() const { return ctas ? E + log_w() + 2 : rows ? E + log_w() + 1 + copies : E + RM + std::max(log_w(), 1) + 1; }
     // Cycles of one exponential of a group alone on its SM sub-partitions
     // (fitted to the spin-1 sweep of 64, one group per SM: 32 lanes, 15
     // instructions, 1,980 cycles; row-aligned at 96 lanes, 3 slots and 4
@@ -499,6 +501,101 @@ inline bool power_pack(const PowSeries& ps, int L, PowLayout* out) {
         for (size_t j = 0; j < sl[k].size(); j++) Ly.merge[j * slots + k] = sl[k][j];
     *out = Ly;
     return true;
+}
+
+// Large systems (k_power_big): the rows dealt to `ctas` CTAs of `threads`
+// lanes, largest first to the CTA with the fewest entries; a row has
+// ceil(entries / E) neighbouring lanes of one warp, E the smallest that lets
+// every CTA hold its rows and its tables in shared memory.  Rows are numbered
+// CTA by CTA (order, first_row).  entry, xoff [cta][E][threads]; mask
+// [cta][threads] lane words.
+constexpr int kPowBigMaxRows = 512, kPowBigMaxCtas = 8;
+constexpr size_t kPowBigSmem = 230 * 1000;   // coefficients, offsets and copies
+// fine steps of the coefficient ring
+inline int pow_big_ring(int ctas) { return ctas == 1 ? 16 : kPowRowsRing; }
+inline bool power_pack_big(const PowSeries& ps, int ctas, int threads, PowLayout* out) {
+    const int M = ps.M, ne = (int)ps.ent.size();
+    PowLayout Ly;
+    std::vector<int> at_mono;
+    if (!pow_monomials(ps, Ly, &at_mono)) return false;
+    const int nm = (int)Ly.mono.size();
+    if (M > kPowBigMaxRows || nm * M >= 65535) return false;
+    std::vector<std::vector<int>> rows(M);
+    for (int i = 0; i < ne; i++) rows[ps.ent[i].row].push_back(i);
+    std::vector<int> ord(M);
+    std::iota(ord.begin(), ord.end(), 0);
+    std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return rows[x].size() > rows[y].size(); });
+    std::vector<long> load(ctas, 0);
+    std::vector<std::vector<int>> mine(ctas);    // rows of each CTA, largest first
+    for (int r : ord) {
+        const int c = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[c] += (long)rows[r].size() + 4;     // a row costs its lanes' last slots too
+        mine[c].push_back(r);
+    }
+    const int warps = threads / 32;
+    for (int E = std::max(1, (ne + ctas * threads - 1) / (ctas * threads));; E++) {
+        if ((size_t)E * threads * 10 + 16 * ((size_t)nm * M + 1) > kPowBigSmem) return false;
+        std::vector<int> first(M, -1);           // a row's first lane in its CTA
+        bool ok = true;
+        int wmax = 1;
+        for (int c = 0; c < ctas && ok; c++) {
+            std::vector<int> used(warps, 0);
+            for (int r : mine[c]) {
+                const int w = std::max(1, ((int)rows[r].size() + E - 1) / E);
+                int k = 0;
+                while (k < warps && used[k] + w > 32) k++;
+                ok = ok && k < warps;
+                if (!ok) break;
+                first[r] = k * 32 + used[k];
+                used[k] += w;
+                wmax = std::max(wmax, w);
+            }
+        }
+        if (!ok) continue;
+        Ly.rows = true;
+        Ly.ctas = ctas;
+        Ly.L = threads;
+        Ly.E = E;
+        Ly.W = wmax;
+        Ly.first_row.assign(1, 0);
+        for (int c = 0; c < ctas; c++) {
+            Ly.order.insert(Ly.order.end(), mine[c].begin(), mine[c].end());
+            Ly.first_row.push_back((int)Ly.order.size());
+        }
+        std::vector<int> pos(M);
+        for (int k = 0; k < M; k++) pos[Ly.order[k]] = k;
+        Ly.entry.assign((size_t)ctas * E * threads, -1);
+        Ly.xoff.assign((size_t)ctas * E * threads, nm * M);
+        Ly.mask.assign((size_t)ctas * threads, (unsigned)M | (1u << 16));
+        for (int c = 0; c < ctas; c++)
+            for (int r : mine[c]) {
+                const int w = std::max(1, ((int)rows[r].size() + E - 1) / E);
+                for (int k = 0; k < w; k++)
+                    Ly.mask[(size_t)c * threads + first[r] + k] =
+                        (unsigned)pos[r] | ((unsigned)w << 16) | ((unsigned)k << 24);
+                for (int i = 0; i < (int)rows[r].size(); i++) {
+                    const size_t slot = ((size_t)c * E + i / w) * threads + first[r] + i % w;
+                    const PowEntry& e = ps.ent[rows[r][i]];
+                    Ly.entry[slot] = rows[r][i];
+                    Ly.xoff[slot] = at_mono[e.mono] * M + pos[e.col];
+                }
+            }
+        *out = Ly;
+        return true;
+    }
+}
+
+// Lanes per CTA for a cluster of `ctas`: enough warps to issue, few enough
+// that the reduction and the barrier stay short (21 levels, 2,000 exponentials:
+// clusters of 4 take 5.8 ms at 256 lanes and 6.9 at 512).
+inline int power_big_threads(int ctas) { return ctas == 1 ? 1024 : ctas <= 2 ? 512 : 256; }
+
+// Cycles of one exponential of a cluster (one CTA per SM): issue of the busiest
+// sub-partition, reduction, and the rest as measured (operand loads of 32 warps
+// for a single CTA, the exchange for the others; 16,100 cycles for 1 CTA, 9,400
+// for 2, 6,000 for 4, 4,900 for 8).
+inline int power_big_cycles(const PowLayout& Ly) {
+    return Ly.L / 128 * Ly.E * 64 + 138 * Ly.log_w() + (Ly.ctas > 1 ? 2700 : 4700);
 }
 
 }  // namespace sss

@@ -62,3 +62,44 @@ def test_power_series_against_oracle(name, K, drives, lanes):
         assert np.abs(tr[b, :s] - ref[b, :s]).max(initial=0.0) <= 1e-12
         assert np.abs(ro[b, :s] - ref[b, :s] @ w).max(initial=0.0) <= 1e-12
         assert not tr[b, s:].any() and not ro[b, s:].any()
+
+
+@pytest.mark.parametrize("B", [1, 5, 20, 40, 80])
+def test_large_system_clusters_against_oracle(B):
+    """The 21-level NV (171 reachable rows) on clusters of 8, 4, 2 and 1 CTAs
+    per trajectory: uneven lengths past the coefficient ring (64 steps; 16 for
+    one CTA), readouts, traces and final states of trajectories from both ends
+    of the batch."""
+    from superspinsim_gb300 import _lib
+    c = load_case("nv21_n441")
+    vm = c["vectorisation_map"]
+    N = vm.shape[0]
+    rng = np.random.default_rng(B)
+    T, F, dt = 2, 40, 2e-10
+    progs = np.zeros((B, 4, 1, 5))
+    progs[:, :, 0, 0] = np.inf
+    progs[:, 0, 0, 2] = 2e-4*rng.uniform(0.5, 1, B)
+    progs[:, 0, 0, 3] = 4.27e9 + rng.uniform(-3e7, 3e7, B)
+    progs[:, 3, 0, 1] = 0.15
+    samples = np.full(B, T, dtype=np.int32)
+    samples[-1] = 1
+    rho = np.zeros((21, 21), complex)
+    for k in range(3, 6):
+        rho[k, k] = 1/3
+    flat = np.stack([oracle.flatten(rho, vm, N)]*B)
+    w = rng.uniform(-1, 1, N)
+    W, nodes = quadrature(2)
+    plan = _lib.Plan(c["generators"], W, nodes)
+    plan.set_batch_config(variant=8)
+    ro, fin, tr = plan.batch(flat, progs, 0.0, dt, T, F, samples=samples, readout_weights=w,
+                             want_final=True, want_trace=True)
+    assert plan.batch_info()["variant"] == 8
+    for b in sorted({0, B//2, B - 1}):
+        _, ref = oracle.simulate(c["generators"], rho[None], 0.0, T*dt + 1e-14, dt, progs[b:b + 1],
+                                 K=2, W=W, nodes=nodes, F=F, vectorisation_map=vm, mode="vector",
+                                 degree=20, flat_out=True)
+        s = samples[b]
+        assert np.abs(fin[b] - ref[0, s - 1]).max() <= 1e-12
+        assert np.abs(tr[b, :s] - ref[0, :s]).max() <= 1e-12
+        assert np.abs(ro[b, :s] - ref[0, :s] @ w).max() <= 1e-12
+        assert not tr[b, s:].any() and not ro[b, s:].any()

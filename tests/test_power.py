@@ -91,17 +91,58 @@ static std::vector<double> run(const PowSeries& ps, const PowLayout& p, int tab,
     return d;
 }
 
+// the same for a cluster's CTAs (k_power_big): rows in the layout's order,
+// the segmented sum over a row's lanes, each row on one CTA and inside a warp
+static std::vector<double> run_big(const PowSeries& ps, const PowLayout& p, int tab,
+                                   const std::vector<double>& a, const std::vector<double>& x) {
+    const int M = ps.M, T = p.L, nm = (int)p.mono.size();
+    const std::vector<double> mv = monomials(p, a);
+    const double* val = &ps.val[tab * ps.ent.size()];
+    std::vector<double> X(nm * M + 1, 0.0), d(M, 0.0);
+    std::vector<int> seen(M, 0);
+    for (int m = 0; m < nm; m++)
+        for (int k = 0; k < M; k++) X[m * M + k] = mv[m] * x[p.order[k]];
+    CHECK((int)p.first_row.size() == p.ctas + 1 && p.first_row.back() == M);
+    for (int c = 0; c < p.ctas; c++) {
+        std::vector<double> s(T);
+        for (int l = 0; l < T; l++)
+            for (int q = 0; q < p.E; q++) {
+                const size_t at = ((size_t)c * p.E + q) * T + l;
+                s[l] += (p.entry[at] < 0 ? 0.0 : val[p.entry[at]]) * X[p.xoff[at]];
+            }
+        auto word = [&](int l) { return p.mask[(size_t)c * T + l]; };
+        for (int o = 1; o < p.W; o <<= 1) {
+            const std::vector<double> t(s);
+            for (int l = 0; l < T; l++) {
+                const int W = (word(l) >> 16) & 0xff, sub = word(l) >> 24;
+                if ((sub & (2 * o - 1)) == 0 && sub + o < W) s[l] = t[l] + t[l + o];
+            }
+        }
+        for (int l = 0; l < T; l++) {
+            const int row = word(l) & 0xffff, W = (word(l) >> 16) & 0xff, sub = word(l) >> 24;
+            if (row == M) continue;
+            CHECK(row >= p.first_row[c] && row < p.first_row[c + 1] && l % 32 - sub + W <= 32);
+            if (sub) continue;
+            d[p.order[row]] = s[l];
+            seen[row]++;
+        }
+    }
+    for (int n : seen) CHECK(n == 1);
+    return d;
+}
+
 int main() {
     std::mt19937_64 rng(7);
     std::uniform_real_distribution<double> u(-1.0, 1.0);
-    int packed = 0;
-    for (int M : {1, 2, 3, 8, 9, 16, 17, 19, 32, 33, 64})
+    int packed = 0, clusters = 0;
+    for (int M : {1, 2, 3, 8, 9, 16, 17, 19, 32, 33, 64, 65, 130})
         for (int n_live : {0, 1, 2})
             for (int n_tab : {1, 3}) {
+                if (M > 64 && (n_live > 1 || n_tab > 1)) continue;
                 std::vector<int> rp(1, 0), col;
                 for (int r = 0; r < M; r++) {
                     for (int c = 0; c < M; c++)
-                        if (c == r || u(rng) > (M > 8 ? 0.8 : 0.0)) col.push_back(c);
+                        if (c == r || u(rng) > (M > 64 ? 0.98 : M > 8 ? 0.8 : 0.0)) col.push_back(c);
                     rp.push_back((int)col.size());
                 }
                 const size_t nnz = col.size();
@@ -146,12 +187,19 @@ int main() {
                         mag[ps.ent[k].row] += std::fabs(ps.val[tab * ps.ent.size() + k]) * m * std::fabs(x[ps.ent[k].col]);
                         n_ent[ps.ent[k].row]++;
                     }
-                    for (int L : {16, 32, 64, 128}) {
+                    // lane counts, and clusters of 1 to 8 CTAs for the large systems
+                    for (int L : {16, 32, 64, 128, -1, -2, -4, -8}) {
                         PowLayout p;
-                        if (!power_pack(ps, L, &p)) continue;
+                        if (L < 0) {
+                            if (M <= 64) continue;
+                            if (!power_pack_big(ps, -L, power_big_threads(-L), &p)) continue;
+                            clusters |= -L;
+                        } else if (!power_pack(ps, L, &p)) {
+                            continue;
+                        }
                         packed++;
-                        CHECK(p.L <= L && (L <= 32 ? p.L == L : p.L % 32 == 0 && p.L >= 64));
-                        const std::vector<double> d = run(ps, p, tab, a, x);
+                        CHECK(L < 0 || (p.L <= L && (L <= 32 ? p.L == L : p.L % 32 == 0 && p.L >= 64)));
+                        const std::vector<double> d = L < 0 ? run_big(ps, p, tab, a, x) : run(ps, p, tab, a, x);
                         for (int r = 0; r < M; r++) {
                             const double tol = 2.0 * (n_ent[r] + 8) * std::ldexp(mag[r], -53) + std::ldexp(xs, -61);
                             if (!(std::fabs((double)(d[r] - ref[r])) <= tol)) {
@@ -163,7 +211,7 @@ int main() {
                     }
                 }
             }
-    CHECK(packed > 100);
+    CHECK(packed > 100 && clusters == 15);
     // too large an exponent is refused
     PowSeries ps;
     CHECK(!power_series(1, {0, 1}, {0}, {{1.5}}, {{0.0}}, {}, {}, &ps));
