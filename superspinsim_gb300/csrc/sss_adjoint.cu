@@ -932,6 +932,37 @@ int adjoint_run_parts(sss_plan* p, int ntraj, const double* d_rho0, int nch, int
     if (per_traj > budget) return fail(SSS_EINVAL, "adjoint states of one trajectory exceed memory");
     const int chunk = (int)std::min<size_t>((size_t)ntraj, budget / per_traj);
 
+    // ---- the forward pass on the power series where that layout fits (its
+    // rows in its own order, which the backward passes read the states in):
+    // the row-part forward of 256 pulse shapes takes as many dependent Horner
+    // terms as a sweep, and every exponential's state is stored either way ----
+    BatchLayout FL;
+    if (p->batch_variant == 0 || p->batch_variant == 8) {
+        struct Flag {
+            sss_plan* p;
+            int variant;
+            explicit Flag(sss_plan* q) : p(q), variant(q->batch_variant) {
+                p->adj_forward = true;
+                p->batch_variant = 0;
+            }
+            ~Flag() {
+                p->adj_forward = false;
+                p->batch_variant = variant;
+            }
+        } flag(p);
+        const int rc = build_layout(p, ntraj, d_rho0, nch, nseg, d_prog, dt, F, {gd}, true, &FL, st);
+        if (rc == SSS_OK && FL.power && FL.M == M) {
+            Ly.newpos = FL.newpos;
+            Ly.row_orig = FL.row_orig;
+        } else if (rc != SSS_OK && rc != SSS_EINVAL) {
+            return rc;
+        } else {
+            FL = BatchLayout();
+            set_error("");
+        }
+    }
+    const BatchLayout& forward = FL.power ? FL : Ly;
+
     // ---- the slot-programmed backward, where the block series fits ----
     if (p->batch_variant != 4 && p->batch_variant != 5 && Ly.degree <= kMaxTaylor) {
         AdjSlotArgs sa{};
@@ -942,7 +973,7 @@ int adjoint_run_parts(sss_plan* p, int ntraj, const double* d_rho0, int nch, int
                                              h_tw, dch, npar, &sa, &BL, &smem, &threads, st);
         if (rc == SSS_OK) {
             PartsForward fw;
-            if (int rc2 = parts_forward_prepare(p, Ly, ntraj, nch, nseg, dt, F, h_rw, {gd},
+            if (int rc2 = parts_forward_prepare(p, forward, ntraj, nch, nseg, dt, F, h_rw, {gd},
                                                 p->w_adjf, &fw, st))
                 return rc2;
             if (int rc2 = p->w_states.ensure(per_traj * chunk)) return rc2;
@@ -1032,7 +1063,7 @@ int adjoint_run_parts(sss_plan* p, int ntraj, const double* d_rho0, int nch, int
 
     // ---- forward tables (the differentiated channel kept live) ----
     PartsForward fw;
-    if (int rc = parts_forward_prepare(p, Ly, ntraj, nch, nseg, dt, F, h_rw, {gd}, p->w_adjf, &fw, st))
+    if (int rc = parts_forward_prepare(p, forward, ntraj, nch, nseg, dt, F, h_rw, {gd}, p->w_adjf, &fw, st))
         return rc;
 
     // ---- backward tables ----

@@ -2077,6 +2077,10 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
     std::vector<int> live, fixed;   // active-generator indices
     for (int gi = 0; gi < Ga; gi++) {
         const int g = active[gi];
+        if (Ly.pw_switch >= 0 && Ly.slot_chan[g] == Ly.pw_switch) {
+            fixed.push_back(gi);   // a value per table
+            continue;
+        }
         (Ly.slot_chan[g] >= 0 && !Ly.chan_const[g] ? live : fixed).push_back(gi);
     }
     if ((int)live.size() > kPowMaxLive) return no("too many varying coefficients");
@@ -2115,15 +2119,19 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
     // double-double; equal ones (the two exponentials of CF4:2) share a table
     using pow_detail::dd;
     std::vector<std::vector<double>> sums, A_hi, A_lo;
-    Ly.pw_tab.assign((size_t)K, 0);
-    for (int e = 0; e < K; e++) {
+    Ly.pw_tab.assign((size_t)K << kMaxQ, 0);
+    const int codes = Ly.pw_switch >= 0 ? 1 << Q : 1;   // the switched channel's value at each node
+    for (int ec = 0; ec < K * codes; ec++) {
+        const int e = ec / codes, code = ec % codes;
         std::vector<double> sv;
         for (int gi : fixed) {
             const int g = active[gi];
-            const double X = Ly.slot_chan[g] < 0 ? 1.0 : Ly.chan_value[g];
+            const bool sw = Ly.pw_switch >= 0 && Ly.slot_chan[g] == Ly.pw_switch;
             dd t{0.0, 0.0};   // rounded once, so that the order of the weights does not show
-            for (int k = 0; k < Q; k++)
+            for (int k = 0; k < Q; k++) {
+                const double X = Ly.slot_chan[g] < 0 ? 1.0 : sw ? Ly.pw_value[(code >> k) & 1] : Ly.chan_value[g];
                 t = pow_detail::dd_add(t, pow_detail::dd_mul({p->W[e * Q + k], 0.0}, {X, 0.0}));
+            }
             sv.push_back(t.hi * h);
         }
         int at = (int)(std::find(sums.begin(), sums.end(), sv) - sums.begin());
@@ -2141,8 +2149,10 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
             A_hi.push_back(hi);
             A_lo.push_back(lo);
         }
-        Ly.pw_tab[e] = at;
+        for (int c = codes > 1 ? code : 0; c < (codes > 1 ? code + 1 : 1 << kMaxQ); c++)
+            Ly.pw_tab[(e << kMaxQ) + c] = at;
     }
+    if (A_hi.size() > (size_t)kPowMaxTables) return no("too many coefficient tables");
     PowSeries ps;
     if (big) {
         // one varying coefficient and one table: with two of either the
@@ -2334,8 +2344,12 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
         a.pw_scale[i] = Ly.pw_scale[i];
     }
     a.pw_sel_ch = -1;
-    for (int e = 0; e < K; e++)
-        for (int c = 0; c < (1 << kMaxQ); c++) a.pw_tab[(e << kMaxQ) + c] = (signed char)Ly.pw_tab[e];
+    if (Ly.pw_switch >= 0) {
+        a.pw_sel_ch = a.n_lch;
+        a.pw_sel_v = Ly.pw_value[1];
+        a.lch_chan[a.n_lch++] = Ly.pw_switch;
+    }
+    for (int i = 0; i < (K << kMaxQ); i++) a.pw_tab[i] = (signed char)Ly.pw_tab[i];
     a.tab_G = p->d.G;
     a.queue = p->w_queue.as<int>();
     p->mk_n_live = a.n_live;
@@ -2567,8 +2581,34 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
     int degree, substeps;
     choose_taylor(beta, p->d.taylor_degree, &degree, &substeps);
 
+    // ---- a forward pass of the adjoint: a channel of two values throughout
+    // (a laser on and off) selects a table of the power series ----
+    for (int c = 0; c < nch && p->adj_forward && !rot && !table; c++) {
+        std::vector<double> vals;
+        bool ok = !chconst[c] && Ly.pw_switch < 0;
+        auto value = [&](double x) {
+            if (std::find(vals.begin(), vals.end(), x) == vals.end()) vals.push_back(x);
+            ok = ok && vals.size() <= 2 && std::isfinite(x);
+        };
+        for (int b = 0; b < ntraj && ok; b++) {
+            const double* seg = h_prog + ((size_t)b * nch + c) * nseg * 5;
+            bool ends = false;
+            for (int q = 0; q < nseg && ok; q++) {
+                if (seg[q * 5] == -INFINITY) continue;
+                ok = seg[q * 5 + 2] == 0.0;
+                value(seg[q * 5 + 1]);
+                ends = ends || seg[q * 5] == INFINITY;
+            }
+            if (!ends) value(0.0);
+        }
+        if (!ok || vals.size() != 2) continue;
+        Ly.pw_switch = c;
+        Ly.pw_value[0] = vals[0];
+        Ly.pw_value[1] = vals[1];
+    }
+
     // ---- samples over which nothing varies: one map per set of values ----
-    if (!table && !rot && allow_register && !force_parts && !p->cols_samples && M <= kConstMaxRows &&
+    if (!p->adj_forward && !table && !rot && allow_register && !force_parts && !p->cols_samples && M <= kConstMaxRows &&
         F * p->d.K >= kConstMinExps)
         constant_layout(p, Ly, h_prog, ntraj, nch, nseg, dt, F);
 
@@ -2583,7 +2623,7 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
             Ly.substeps = 1;
             return SSS_OK;
         }
-        if (power_asked) return rc;
+        if (power_asked || p->adj_forward) return rc;
     }
 
     // ---- lanes per trajectory ----
@@ -3325,7 +3365,7 @@ int batch_launch(sss_plan* p, double* d_state, const double* d_prog, const int* 
 int parts_forward_prepare(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int nseg,
                           double dt, int F, const double* h_rw, const std::vector<int>& keep_live,
                           DevBuf& tables, PartsForward* fw, cudaStream_t st) {
-    if (!Ly.parts) return fail(SSS_EINVAL, "not a row-part layout");
+    if (!Ly.parts && !Ly.power) return fail(SSS_EINVAL, "not a row-part or power-series layout");
     BatchArgs a{};
     size_t smem = 0;
     if (int rc = make_args(p, Ly, ntraj, nch, nseg, dt, F, h_rw, keep_live, tables, &a, &smem, st))
@@ -3337,6 +3377,10 @@ int parts_forward_prepare(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch
     fw->C = Ly.C;
     fw->P = Ly.P;
     fw->threads = Ly.threads;
+    fw->power = Ly.power;
+    fw->E = Ly.E;
+    fw->RM = Ly.pl.RM;
+    fw->ctas = Ly.pl.ctas;
     return SSS_OK;
 }
 
@@ -3360,6 +3404,9 @@ int parts_forward_launch(sss_plan* p, const PartsForward& fw, int ntraj, double*
     a.states = d_states;
     a.st_steps = (long)T * a.F;
     SSS_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(int), st));
+    if (fw.power)
+        return fw.ctas ? launch_power_big(p, fw.ctas, a, fw.threads, fw.smem, st)
+                       : launch_power(p, fw.L, fw.E, fw.RM, a, fw.threads, fw.smem, st);
     switch (fw.L) {
         case 8: return launch_parts<8>(p, fw.C, fw.P, a, fw.threads, fw.smem, st);
         case 16: return launch_parts<16>(p, fw.C, fw.P, a, fw.threads, fw.smem, st);

@@ -98,7 +98,11 @@ struct BatchLayout {
     PowLayout pl;
     std::vector<int> pw_live;
     double pw_scale[kPowMaxLive] = {};
-    std::vector<int> pw_tab;
+    std::vector<int> pw_tab;                 // [exponential << kMaxQ + code of the switched channel]
+    // the switched channel of a forward pass of the adjoint, -1: none, and its
+    // two values
+    int pw_switch = -1;
+    double pw_value[2] = {};
     // samples over which every live channel is constant (sss_constant.h): the
     // live program channels, the sets of their values, and the maps minus the
     // identity [set][hi, lo][column][row], rows in reachable order
@@ -185,6 +189,10 @@ struct sss_plan {
     // reads the device copies back)
     const double *host_rho0 = nullptr, *host_prog = nullptr;
     sss::DevBuf w_cols_tables, w_cols_queue;
+    // the adjoint's forward pass being laid out on the power series: every
+    // exponential's state is stored, and a channel of two values throughout the
+    // programs (they cannot change before the launch) selects a table
+    bool adj_forward = false;
     int launch_active = 0;       // trajectories with work in the next launch (0: the batch)
     // prepared batch (sss_batch_prepare -> sss_batch_launch): one kernel
     // layout per phase -- a single phase, or with uneven lengths and
@@ -291,6 +299,8 @@ struct PartsForward {
     alignas(16) unsigned char args[2048];
     size_t smem = 0;
     int L = 0, C = 0, P = 0, threads = 0;
+    bool power = false;   // the power-series kernels: E slots, RM merge slots, CTAs of a cluster
+    int E = 0, RM = 0, ctas = 0;
 };
 // Build the device tables of a row-part layout into `tables` and the
 // forward kernel's arguments.  Generators in `keep_live` are never folded
