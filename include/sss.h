@@ -113,7 +113,11 @@ int sss_plan_set_rotating(sss_plan* plan, const double* generators_nodes,
  *          row order (sample t, node k at fine step r in row
  *          (r*T + t)*Q + k), or NULL
  *   out:   ntraj*T*N  state after each of the T output samples
- * Output sample t is at t0 + dt*(t+1); each spans F fine steps of dt/F. */
+ * Output sample t is at t0 + dt*(t+1); each spans F fine steps of dt/F.
+ * With SSS_EXPM_TAYLOR the samples' propagators are built column by column by
+ * the batched kernels on the rows reachable from rho0; SSS_EXPM_REFERENCE,
+ * unitary mode and exponents too large for the Taylor action build them by
+ * dense products, as sss_simulate_device always does. */
 int sss_simulate(sss_plan* plan, int ntraj, const double* rho0, int nch,
                  int nseg, const double* programs, const double* coeff_table,
                  double t0, double dt, int T, int F, double* out,

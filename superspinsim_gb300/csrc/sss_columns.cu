@@ -38,6 +38,7 @@ int batch_columns_launch(sss_plan* p, const BatchLayout& Ly, const BatchArgs& a,
 namespace {
 
 constexpr int kBlock = 16;          // samples per block of the chain
+constexpr int kMaxTerms = 256;      // Taylor terms per exponential (dense products cost about 400)
 constexpr int kLanesPerRow = 8;     // lanes of a matrix row in the chain kernels
 
 struct ChainArgs {
@@ -295,6 +296,10 @@ int columns_run(sss_plan* p, int ntraj, const double* h_rho0, const double* d_rh
         return rc;
     const int M = Ly.M;
     if (M == 0 || !(Ly.slots || Ly.power)) return fail(SSS_EINVAL, "no column layout");
+    // an exponent so large that the Taylor action takes hundreds of terms (its
+    // sub-steps end at 1,024) is the dense path's: scaling and squaring
+    if (Ly.slots && (long)Ly.degree * Ly.substeps > kMaxTerms)
+        return fail(SSS_EINVAL, "the exponent is too large for the Taylor action");
     BatchArgs a{};
     size_t smem = 0;
     if (int rc = batch_columns_args(p, Ly, ntraj, nch, nseg, dt, F, p->w_cols_tables, &a, &smem, st)) return rc;

@@ -155,3 +155,27 @@ def test_columns_leave_a_prepared_batch_alone():
     after = plan.batch_info()
     for key in ("lanes", "degree", "rows", "nnz", "variant", "live_generators", "live_nnz"):
         assert after[key] == info[key]
+
+
+@pytest.mark.parametrize("dt", [1e-9, 1e-7, 1e-5])
+def test_large_steps_keep_the_dense_exponential(dt):
+    """One fine step per sample of 1 ns to 10 us (1-norms of the exponent of 20
+    to 200,000) under a constant field: the matrix exponential, by sub-steps of
+    the Taylor action or, beyond its range, by the dense path's scaling and
+    squaring (which doubles the rounding once per squaring: 2^-53 times the
+    norm)."""
+    from scipy.linalg import expm
+    c = load_case("spin1_c1")
+    vm = c["vectorisation_map"]
+    plan, W, nodes = _plan(c, 1, dt, 1, False, True)
+    prog = np.zeros((1, 4, 1, 5))
+    prog[:, :, 0, 0] = np.inf
+    prog[0, 0, 0, 1] = 1e-4
+    rho = np.diag([0.25, 0.75, 0.0]).astype(complex)
+    flat = oracle.flatten(rho, vm, vm.shape[0])
+    out = plan.simulate(flat[None], prog, 0.0, dt, 3, 1)[0]
+    L = (c["generators"][0] + 1e-4*c["generators"][1])*dt
+    x, E = flat, expm(L)
+    for t in range(3):
+        x = E @ x
+        assert np.abs(out[t] - x).max() <= 1e-12 + 64*2.0**-53*np.abs(L).sum(0).max()
