@@ -64,7 +64,7 @@ def test_power_series_against_oracle(name, K, drives, lanes):
         assert not tr[b, s:].any() and not ro[b, s:].any()
 
 
-@pytest.mark.parametrize("B", [1, 5, 20, 40, 80])
+@pytest.mark.parametrize("B", [1, 5, 20, 40, 80, 170])
 def test_large_system_clusters_against_oracle(B):
     """The 21-level NV (171 reachable rows) on clusters of 8, 4, 2 and 1 CTAs
     per trajectory: uneven lengths past the coefficient ring (64 steps; 16 for
@@ -103,3 +103,32 @@ def test_large_system_clusters_against_oracle(B):
         assert np.abs(tr[b, :s] - ref[0, :s]).max() <= 1e-12
         assert np.abs(ro[b, :s] - ref[0, :s] @ w).max() <= 1e-12
         assert not tr[b, s:].any() and not ro[b, s:].any()
+
+
+@pytest.mark.parametrize("name,B", [("spin1_c1", 5), ("nv7_n19", 700), ("nv21_n441", 3)])
+def test_chunks_and_graph_replay(name, B):
+    """Chunked launches and their CUDA graph give the one-shot run bit for bit
+    on the row-aligned, the 32-lane and the cluster kernels."""
+    torch = pytest.importorskip("torch")
+    from superspinsim_gb300.sweep import ChunkedRun, Sweep
+    c = load_case(name)
+    vm = c["vectorisation_map"]
+    n = int(vm[:, 0].max()) + 1
+    rng = np.random.default_rng(4)
+    T, F, dt = 5, 9, 1e-10
+    progs = np.zeros((B, 4, 1, 5))
+    progs[:, :, 0, 0] = np.inf
+    progs[:, 0, 0, 2] = 1e-4*rng.uniform(0.5, 1, B)
+    progs[:, 0, 0, 3] = 3.0e9 + rng.uniform(-3e7, 3e7, B)
+    rho = np.zeros((n, n), complex)
+    rho[1, 1] = 1.0
+    w = rng.uniform(-1, 1, vm.shape[0])
+    sw = Sweep(c["generators"], vm, number_of_exponentials=2, number_of_fine_divisions=F)
+    one = sw.run(rho, progs, 0.0, T*dt + 1e-14, dt, readout_weights=w, final_state=True)
+    assert sw.info()["variant"] == 8
+    for run in (ChunkedRun(sw, rho, progs, 0.0, dt, T, readout_weights=w).run(chunk=2),
+                ChunkedRun(sw, rho, progs, 0.0, dt, T, readout_weights=w).capture(chunk=3).replay()):
+        torch.cuda.synchronize()
+        r = run.results()
+        assert np.array_equal(r["readout"], one["readout"])
+        assert np.array_equal(r["final"], one["final"])
