@@ -2167,6 +2167,7 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
         while (ctas > 1 && n > power_big_resident(ctas)) ctas /= 2;
         const double slots = (double)((nnz + M + 127) / 128), per_sm = std::ceil((double)n / p->num_sms);
         const double taylor = horner_terms * std::max(105.0 * slots + 500.0, 64.0 * slots * per_sm);
+        const int n_chan = (int)live.size() + (Ly.pw_switch >= 0);
         std::vector<double> key{(double)M};
         key.insert(key.end(), row_ptr.begin(), row_ptr.end());
         key.insert(key.end(), col.begin(), col.end());
@@ -2182,8 +2183,15 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
             p->series_memo[key] = ps;
         }
         PowLayout pl;
-        if (!power_pack_big(ps, ctas, power_big_threads(ctas), &pl)) return no("no layout fits");
-        if (!asked && power_big_cycles(pl) * (ctas > 1 ? 1.0 : per_sm) > taylor)
+        // tables that outgrow a CTA's shared memory go to twice as many CTAs,
+        // whose clusters then take the trajectories in turn
+        while (!power_pack_big(ps, ctas, power_big_threads(ctas), &pl, K, Q, n_chan)) {
+            ctas *= 2;
+            if (ctas > kPowBigMaxCtas) return no("no layout fits");
+        }
+        const int resident = power_big_resident(ctas);
+        if (resident < 1) return no("no cluster fits on the GPU");
+        if (!asked && power_big_cycles(pl) * std::ceil((double)n / resident) > taylor)
             return no("the Taylor action is cheaper");
         for (int i = 0; i < kLaneCounts; i++) p->auto_cost[i] = p->auto_chain[i] = 0.0;
         Ly.power = true;
@@ -2207,6 +2215,9 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
     if (ps.ent.empty()) return no("nothing to do");
     // lanes: the automatic rule on the costs of one exponential (two CTA
     // barriers where a group is wider than a warp)
+    // (a layout whose CTA outgrows shared memory does not count)
+    const int n_chan = (int)live.size() + (Ly.pw_switch >= 0);
+    auto cta_threads = [&](int L) { return std::max(L, p->batch_threads > 0 ? std::min(p->batch_threads, 128) : 32); };
     PowLayout lay[kLaneCounts];
     double cost[kLaneCounts] = {}, chain[kLaneCounts] = {}, floor_cost[kLaneCounts] = {};
     for (int i = 0; i < kLaneCounts; i++) {
@@ -2217,6 +2228,7 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
                                                 (L > 32 ? 1.0 : 0.0));
         if (p->batch_lanes > 0 && p->batch_lanes != L) continue;
         if (!power_pack(ps, L, &lay[i])) continue;
+        if (power_smem(lay[i], M, K, Q, n_chan, L > 32 ? 1 : cta_threads(L) / L) > kPowSmem) continue;
         // issue figure (the CTA barrier and fewer groups to fill it cost a
         // group wider than a warp about six instructions: 7-level sweep of
         // 1024, 128 lanes 60 ms where their 13 instructions alone make 44)
@@ -2245,8 +2257,7 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
         p->auto_cost[i] = cost[i];
         p->auto_chain[i] = chain[i];
     }
-    int threads = std::max(L, p->batch_threads > 0 ? std::min(p->batch_threads, 128) : 32);
-    if (L > 32) threads = lay[li].L;
+    const int threads = L > 32 ? lay[li].L : cta_threads(L);
     if (L <= 32 && threads % L) return no("CTA size must be a multiple of the lanes per trajectory");
     Ly.power = true;
     Ly.ps = ps;
@@ -2356,18 +2367,7 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     p->mk_live_nnz = (int)ne;
     p->last_bank_before = p->last_bank_after = 0;
     *out = a;
-    if (pl.ctas) {
-        *smem = sizeof(double) * (2 * (size_t)(a.pw_mono * M + 1) +
-                                  (size_t)pow_big_ring(pl.ctas) * (Q * a.n_lch + K * a.pw_mono) + a.pw_mono) +
-                (sizeof(double) + sizeof(unsigned short)) * (size_t)E * L;
-        if (*smem > 226 * 1024) return fail(SSS_EINVAL, "power-series kernel: shared memory per CTA too large");
-        return SSS_OK;
-    }
-    const size_t ring = (size_t)(pl.rows ? kPowRowsRing : kRing);
-    const size_t per_slot = ((size_t)(pl.rows ? 2 * (a.pw_mono * M + 1) : M + 1 + pl.n_part + 1) +
-                             ring * (Q * a.n_lch + K * a.pw_mono) + a.pw_mono + ring * K / 2) | 1;
-    *smem = sizeof(double) * (pl.rows ? 1 : Ly.threads / L) * per_slot;
-    if (*smem > 227 * 1024) return fail(SSS_EINVAL, "power-series kernel: shared memory per CTA too large");
+    *smem = power_smem(pl, M, K, Q, a.n_lch, pl.rows ? 1 : Ly.threads / L);
     return SSS_OK;
 }
 

@@ -33,6 +33,8 @@
 namespace sss {
 namespace {
 
+static_assert(kRing == kPowRing, "power_smem counts the ring");
+
 // A trajectory taken from the queue: its program's index, output samples and,
 // for propagator columns, the column.
 struct PowTrajectory {

@@ -61,6 +61,7 @@ inline int pow_pick(const int (&table)[N], int want) {
 // the whole group waits for, is paid every 64 steps (28.4 against 27.1 ms on
 // the spin-1 sweep of 64 with 16 steps).
 constexpr int kPowRowsRing = 64;
+constexpr int kPowRing = 16;       // and of the other kernels (kRing)
 constexpr int kPowRowLanes = 16;   // lanes of a row, at most
 
 struct PowEntry {
@@ -336,6 +337,26 @@ struct PowLayout {
 
 inline int pow_sequences(int E) { return E >= 12 ? 2 : 1; }
 
+// fine steps of the coefficient ring of a cluster of `ctas`
+inline int pow_big_ring(int ctas) { return ctas == 1 ? kPowRing : kPowRowsRing; }
+
+// Dynamic shared memory of one CTA of a layout on M rows: `groups` groups of
+// state (or copies), partial sums and ring, for K exponentials of Q nodes on
+// n_chan channels; and a cluster's coefficients and operand offsets.  Every
+// layout is checked against kPowSmem when it is chosen, so that one that does
+// not fit gives way to another.
+constexpr size_t kPowSmem = 226 * 1024;   // 227 KB less the kernels' static arrays
+inline size_t power_smem(const PowLayout& Ly, int M, int K, int Q, int n_chan, int groups) {
+    const size_t nm = Ly.mono.size(), copies = 2 * (nm * M + 1);
+    if (Ly.ctas)
+        return sizeof(double) * (copies + (size_t)pow_big_ring(Ly.ctas) * (Q * n_chan + K * nm) + nm) +
+               (sizeof(double) + sizeof(unsigned short)) * (size_t)Ly.E * Ly.L;
+    const size_t ring = (size_t)(Ly.rows ? kPowRowsRing : kPowRing);
+    const size_t per_group = ((Ly.rows ? copies : (size_t)(M + 1 + Ly.n_part + 1)) +
+                              ring * (Q * n_chan + K * nm) + nm + ring * K / 2) | 1;
+    return sizeof(double) * groups * per_group;
+}
+
 // The monomials in use and their factors, by degree; at_mono: the value of
 // each of the series' monomials.  False when the ring cannot hold them.
 inline bool pow_monomials(const PowSeries& ps, PowLayout& Ly, std::vector<int>* at_mono) {
@@ -506,14 +527,13 @@ inline bool power_pack(const PowSeries& ps, int L, PowLayout* out) {
 // Large systems (k_power_big): the rows dealt to `ctas` CTAs of `threads`
 // lanes, largest first to the CTA with the fewest entries; a row has
 // ceil(entries / E) neighbouring lanes of one warp, E the smallest that lets
-// every CTA hold its rows and its tables in shared memory.  Rows are numbered
+// every CTA hold its rows; false when its tables then outgrow shared memory
+// (K exponentials of Q nodes on n_chan channels).  Rows are numbered
 // CTA by CTA (order, first_row).  entry, xoff [cta][E][threads]; mask
 // [cta][threads] lane words.
 constexpr int kPowBigMaxRows = 512, kPowBigMaxCtas = 8;
-constexpr size_t kPowBigSmem = 230 * 1000;   // coefficients, offsets and copies
-// fine steps of the coefficient ring
-inline int pow_big_ring(int ctas) { return ctas == 1 ? 16 : kPowRowsRing; }
-inline bool power_pack_big(const PowSeries& ps, int ctas, int threads, PowLayout* out) {
+inline bool power_pack_big(const PowSeries& ps, int ctas, int threads, PowLayout* out, int K = 2, int Q = 2,
+                           int n_chan = 1) {
     const int M = ps.M, ne = (int)ps.ent.size();
     PowLayout Ly;
     std::vector<int> at_mono;
@@ -534,7 +554,10 @@ inline bool power_pack_big(const PowSeries& ps, int ctas, int threads, PowLayout
     }
     const int warps = threads / 32;
     for (int E = std::max(1, (ne + ctas * threads - 1) / (ctas * threads));; E++) {
-        if ((size_t)E * threads * 10 + 16 * ((size_t)nm * M + 1) > kPowBigSmem) return false;
+        Ly.ctas = ctas;
+        Ly.L = threads;
+        Ly.E = E;
+        if (power_smem(Ly, M, K, Q, n_chan, 1) > kPowSmem) return false;
         std::vector<int> first(M, -1);           // a row's first lane in its CTA
         bool ok = true;
         int wmax = 1;
@@ -553,9 +576,6 @@ inline bool power_pack_big(const PowSeries& ps, int ctas, int threads, PowLayout
         }
         if (!ok) continue;
         Ly.rows = true;
-        Ly.ctas = ctas;
-        Ly.L = threads;
-        Ly.E = E;
         Ly.W = wmax;
         Ly.first_row.assign(1, 0);
         for (int c = 0; c < ctas; c++) {
