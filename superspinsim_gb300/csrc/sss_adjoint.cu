@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256) k_adjoint(const AdjArgs a) {
 
 template <int L>
 int launch_adj(sss_plan* p, const AdjArgs& a, int threads, size_t smem, int grid, cudaStream_t st) {
-    SSS_CUDA(cudaFuncSetAttribute(k_adjoint<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(k_adjoint<L>)) return rc;
     k_adjoint<L><<<grid, threads, smem, st>>>(a);
     SSS_CUDA(cudaGetLastError());
     (void)p;
@@ -696,7 +696,7 @@ template <int L>
 int launch_adj_parts(sss_plan* p, int C, int P, const AdjPartsArgs& a, int threads, size_t smem,
                      cudaStream_t st) {
     auto go = [&](auto kern) -> int {
-        SSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (int rc = allow_smem(kern)) return rc;
         int per_sm = 0;
         SSS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
         if (per_sm < 1) return fail(SSS_EINVAL, "adjoint kernel does not fit on an SM");

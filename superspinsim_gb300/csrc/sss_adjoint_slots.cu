@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256, 1) k_adjoint_slots(const AdjSlotArgs a) {
 template <class Kern>
 int launch_adj(sss_plan* p, Kern kern, const AdjSlotArgs& a, int threads, int slots_per_cta,
                size_t smem, cudaStream_t st) {
-    SSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(kern)) return rc;
     int per_sm = 0;
     SSS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     if (per_sm < 1) return fail(SSS_EINVAL, "adjoint kernel does not fit on an SM");

@@ -193,7 +193,7 @@ constexpr int kPhasedShapeCount = (int)(sizeof(kPhasedShapes) / sizeof(kPhasedSh
 template <class Kern>
 inline int launch(sss_plan* p, Kern kern, const BatchArgs& a, int threads, int slots_per_cta,
            size_t smem, cudaStream_t st) {
-    SSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(kern)) return rc;
     int per_sm = 0;
     SSS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     if (per_sm < 1) return fail(SSS_EINVAL, "batched kernel does not fit on an SM");

@@ -337,7 +337,7 @@ int columns_run(sss_plan* p, int ntraj, const double* h_rho0, const double* d_rh
     const int nio = p->state_in();
     const int threads = (M * kLanesPerRow + 31) / 32 * 32;
     const size_t psmem = 3 * per_sample;
-    SSS_CUDA(cudaFuncSetAttribute(k_block_product, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem));
+    if (int rc = allow_smem(k_block_product)) return rc;
     int launches = 0;
     for (int b = 0; b < ntraj; b += nb) {
         const int n = std::min(nb, ntraj - b);

@@ -40,6 +40,23 @@ int cuda_fail(cudaError_t e, const char* what);
         if (e_ != cudaSuccess) return sss::cuda_fail(e_, #call); \
     } while (0)
 
+// Lets `kern` be launched with as much dynamic shared memory as the device gives
+// a block.  The limit belongs to the function and so to the whole process: every
+// caller sets it to that maximum and none to its own launch's size, which would
+// make a larger launch of another thread fail.
+template <class Kern>
+inline int allow_smem(Kern kern) {
+    cudaFuncAttributes fa;
+    int dev = 0, most = 0;
+    SSS_CUDA(cudaFuncGetAttributes(&fa, kern));
+    SSS_CUDA(cudaGetDevice(&dev));
+    SSS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    most -= (int)fa.sharedSizeBytes;
+    if (fa.maxDynamicSharedSizeBytes < most)
+        SSS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return 0;
+}
+
 // Device buffer that grows on demand and is owned by a plan.
 struct DevBuf {
     void* p = nullptr;

@@ -166,7 +166,7 @@ int power_big_resident(int ctas) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int active = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+    if (allow_smem(kernel) ||
         cudaOccupancyMaxActiveClusters(&active, kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -176,7 +176,7 @@ int power_big_resident(int ctas) {
 
 int launch_power_big(sss_plan* p, int ctas, const BatchArgs& a, int threads, size_t smem, cudaStream_t st) {
     const auto kernel = pow_big_ring(ctas) == kRing ? k_power_big<kRing> : k_power_big<kPowRowsRing>;
-    SSS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(kernel)) return rc;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
