@@ -19,7 +19,8 @@
 // entries, because an entry's rounding is the same at every step: 2^-58 at
 // an entry of 0.05 would be a drift of 3e-12 over 800,000 exponentials.
 // Entries are dropped, smallest first, while the dropped sum of every
-// column stays below a bound (kPowDrop).
+// column stays below a bound (kPowDrop), and degrees are left out once all of
+// the next one is below it.
 //
 // power_pack() deals the entries to the lanes of a group.
 #pragma once
@@ -32,8 +33,8 @@
 namespace sss {
 
 constexpr int kPowMaxLive = 2;     // varying coefficients in the series
-constexpr int kPowMaxDegree = 8;   // total degree
-constexpr int kPowMaxMono = 24;    // monomial values per exponential (kernel ring)
+constexpr int kPowMaxDegree = 9;   // total degree
+constexpr int kPowMaxMono = 28;    // monomial values per exponential (kernel ring; degree 6 of two)
 // Entries and low parts below 2^-62 of the state are dropped: the 16,000
 // exponentials of the 1024-frequency sweep keep the Taylor action's error of
 // 3e-15 (2^-58 drops 10 % more and drifts to 1.2e-13).  A propagator column is
@@ -135,8 +136,11 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
     }
     for (int g = 0; g < n_live; g++) b += rho[g] * norm1(G[g]);
     if (!(b <= 0.25)) return false;
+    // the terms left out are below what may be dropped, as the entries are: they
+    // are missing at every exponential too
+    const double drop = std::min(kPowDrop, kPowDropSmall * std::pow(x + b, 1.5));
     int deg = 0;
-    for (double t = b * std::exp(x); n_live && t > std::ldexp(1.0, -60); deg++) t *= b / (deg + 2);
+    for (double t = b * std::exp(x); n_live && t > drop; deg++) t *= b / (deg + 2);
     if (deg > kPowMaxDegree) return false;
     // monomials by total degree
     PowSeries& ps = *out;
@@ -231,7 +235,6 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
     }
     // keep, per column, all but the smallest entries (by their largest value
     // over the tables) whose sum stays below the bound
-    const double drop = std::min(kPowDrop, kPowDropSmall * std::pow(x + b, 1.5));
     std::vector<char> keep((size_t)nm * MM, 0);
     std::vector<std::pair<double, size_t>> colv;
     std::vector<double> size(nm, 1.0);   // largest value of each monomial
