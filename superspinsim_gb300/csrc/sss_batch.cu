@@ -2607,8 +2607,9 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
         Ly.pw_value[1] = vals[1];
     }
 
-    // ---- samples over which nothing varies: one map per set of values ----
-    if (!p->adj_forward && !table && !rot && allow_register && !force_parts && !p->cols_samples && M <= kConstMaxRows &&
+    // ---- samples over which nothing varies: one map per set of values (a plan
+    // that fixes its Taylor degree steps them at that degree like the others) ----
+    if (!p->adj_forward && p->d.taylor_degree == 0 && !table && !rot && allow_register && !force_parts && !p->cols_samples && M <= kConstMaxRows &&
         F * p->d.K >= kConstMinExps)
         constant_layout(p, Ly, h_prog, ntraj, nch, nseg, dt, F);
 
