@@ -2049,6 +2049,17 @@ static void constant_tables(const BatchLayout& Ly, const std::vector<int>& lch, 
                     Ly.cs_map[((size_t)k * M + c) * M + r];
 }
 
+// ... and their kernel arguments (after dt and F).
+static void constant_args(const sss_plan* p, const BatchLayout& Ly, const double* val, const double* map,
+                          BatchArgs& a) {
+    a.n_const = (int)Ly.cs.size();
+    a.cset = val;
+    a.cmat = map;
+    const auto node = std::minmax_element(p->nodes, p->nodes + p->d.Q);
+    a.noff_min = (a.dt * *node.first) / a.F;
+    a.noff_max = (a.dt * *node.second) / a.F;
+}
+
 // The power-series layout of a batch (sss_power.h) on the pruned pattern
 // row_ents: the series of every distinct constant part over the exponentials
 // of a step, packed for the lane count the automatic rule takes on its costs
@@ -2346,9 +2357,7 @@ static int make_power_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nc
     }
     a.n_live = (int)Ly.pw_live.size();
     a.n_lch = a.n_live;
-    a.n_const = (int)Ly.cs.size();
-    a.cset = dv + o_cval;
-    a.cmat = dv + o_cmap;
+    constant_args(p, Ly, dv + o_cval, dv + o_cmap, a);
     for (int i = 0; i < a.n_live; i++) {
         a.live_ch[i] = i;
         a.lch_chan[i] = lch[i];
@@ -3028,11 +3037,7 @@ static int make_args(sss_plan* p, const BatchLayout& Ly, int ntraj, int nch, int
         p->mk_n_live = (int)live.size();
         p->mk_live_nnz = lnnz;
     }
-    if (constants) {
-        a.n_const = (int)Ly.cs.size();
-        a.cset = dv + o_cval;
-        a.cmat = dv + o_cmap;
-    }
+    if (constants) constant_args(p, Ly, dv + o_cval, dv + o_cmap, a);
     if (Ly.slots) {
         a.S = Ly.S;
         a.bar_at = Ly.bar_at;

@@ -93,6 +93,7 @@ struct BatchArgs {
     // constant samples (sss_constant.h): sets, their values [set][live channel]
     // and maps [set][hi, lo][column][row]
     int n_const;
+    double noff_min, noff_max; // smallest and largest of noff
     const double *cset, *cmat;
     // propagator columns: a trajectory is column (index mod cols) of the
     // propagators of a run of col_len samples, col_runs runs per trajectory
@@ -111,14 +112,14 @@ __device__ __forceinline__ void note_nonfinite(const BatchArgs& a, double x, int
 
 // The set of constant values that the live channels hold over all of output
 // sample t, or -1: each in one segment of zero amplitude (or past its last)
-// from the first node of the sample to its last, at values of one of the
-// batch's sets.  Values no set holds (programs changed after the batch was
+// from the earliest node of the sample to its latest (a plan's nodes come in any
+// order), at values of one of the batch's sets.  Values no set holds (programs changed after the batch was
 // prepared) step as any others.
 __device__ __forceinline__ int constant_set(const BatchArgs& a, const double* prog, int t) {
     if (!prog) return -1;
     const double base = __dmul_rn(a.dt, (double)t);
-    const double t_first = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff)), base), __ldg(a.noff));
-    const double t_last = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff + a.F - 1)), base), __ldg(a.noff + a.Q - 1));
+    const double t_first = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff)), base), a.noff_min);
+    const double t_last = __dadd_rn(__dadd_rn(__dadd_rn(a.t0, __ldg(a.toff + a.F - 1)), base), a.noff_max);
     unsigned left = (1u << a.n_const) - 1u;
     for (int ci = 0; ci < a.n_lch; ci++) {
         const int ch = a.lch_chan[ci];
