@@ -23,6 +23,7 @@
 // must not read its inputs on the host) and what no layout fits keep the
 // dense path.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "sss_batch_args.cuh"
@@ -260,6 +261,11 @@ int columns_run(sss_plan* p, int ntraj, const double* h_rho0, const double* d_rh
     const int N = p->d.N;
     if (N > kPlainMaxN || p->u_n || p->d.expm != SSS_EXPM_TAYLOR || p->d.taylor_degree > 0)
         return fail(SSS_EINVAL, "not a run by columns");
+    // a coefficient that is not finite is the dense path's: it reports the NaN
+    // that its generator makes of every state, also of the rows it does not move
+    // (1e100: the cosine's argument then stays finite)
+    for (size_t i = 0, n = h_prog ? (size_t)ntraj * nch * nseg * 5 : 0; i < n; i++)
+        if (i % 5 && !(std::fabs(h_prog[i]) <= 1e100)) return fail(SSS_EINVAL, "a coefficient is not finite");
     // the plan's batched configuration and report stay as they are
     struct Saved {
         sss_plan* p;
