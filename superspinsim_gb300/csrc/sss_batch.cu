@@ -2541,12 +2541,8 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
     Ly.active = active;
     if (M == 0) return SSS_OK;
     if (p->cols_samples) {
-        // as many columns as fill the SM sub-partitions with four warps of
-        // 8-lane groups each; fewer, longer runs past that (the states inside
-        // a run need no chain)
-        const long want = 16L * 4 * p->num_sms;
-        p->cols_len = (int)std::max(1L, (p->cols_samples * M + want - 1) / want);
-        p->auto_lanes_ntraj = (int)std::min(1L << 30, (p->cols_samples + p->cols_len - 1) / p->cols_len * M);
+        p->cols = columns_cut(ntraj, T_tab, M, p->num_sms);
+        p->auto_lanes_ntraj = (int)std::min(1L << 30, p->cols.runs * M);
     }
     if (M > 65534) return fail(SSS_EINVAL, "batched kernel supports at most 65534 reachable rows");
     std::vector<int> pos_of_orig(N, -1);

@@ -38,10 +38,9 @@ int batch_columns_launch(sss_plan* p, const BatchLayout& Ly, const BatchArgs& a,
 
 namespace {
 
-constexpr int kBlock = 16;          // samples per block of the chain
+constexpr int kBlock = kColBlock;   // runs per block of the chain
 constexpr int kMaxTerms = 256;      // Taylor terms per exponential (dense products cost about 400)
 constexpr int kLanesPerRow = 8;     // lanes of a matrix row in the chain kernels
-constexpr int kMaxGridY = 65535;    // blocks in a grid's y dimension
 
 struct ChainArgs {
     int M, N, n_full, T, len, t_begin;   // samples in this chunk, per run; global first sample
@@ -310,15 +309,9 @@ int columns_run(sss_plan* p, int ntraj, const double* h_rho0, const double* d_rh
     BatchArgs a{};
     size_t smem = 0;
     if (int rc = batch_columns_args(p, Ly, ntraj, nch, nseg, dt, F, p->w_cols_tables, &a, &smem, st)) return rc;
-    const int len = p->cols_len;
-    // chunks of samples (whole blocks) and trajectories that keep the
-    // propagators under 2 GiB; the chain kernels have the trajectories in
-    // grid y, 65,535 at most
+    // launches of whole blocks of samples, or of whole trajectories
+    const int len = p->cols.len, step = kBlock * len, Tc = std::min(T, p->cols.samples), nb = p->cols.traj;
     const size_t per_sample = sizeof(double) * (size_t)M * M;
-    const int step = kBlock * len;
-    const size_t cap = (2ull << 30) / per_sample;
-    int Tc = T, nb = (int)std::min<size_t>(std::min(ntraj, kMaxGridY), std::max<size_t>(1, cap / std::max(1, T)));
-    if (nb == 1 && (size_t)T > cap) Tc = std::max(step, (int)(cap / step) * step);
     const int blocks_c = (Tc + step - 1) / step;
     const bool direct = !p->rotating && !p->n_full;
     if (int rc = p->w_prop.ensure(per_sample * Tc * nb)) return rc;

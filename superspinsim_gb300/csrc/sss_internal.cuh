@@ -9,6 +9,7 @@
 
 #include "sss.h"
 #include "sss_lanes.h"
+#include "sss_columns.h"
 #include "sss_constant.h"
 #include "sss_power.h"
 
@@ -198,10 +199,10 @@ struct sss_plan {
     double auto_cost[sss::kLaneCounts] = {};  // last automatic layout: cost per lane count 8..256
     double auto_chain[sss::kLaneCounts] = {}; // and its chain figures (auto_lane_count)
     // a run by propagator columns being laid out or launched (sss_columns.cu):
-    // its samples over all trajectories (0: not one) and the samples per run;
-    // its launches record no timing events
+    // its samples over all trajectories (0: not one) and its launches, which
+    // record no timing events
     long cols_samples = 0;
-    int cols_len = 1;
+    sss::ColumnsCut cols;
     // the inputs of the call on the host, where it has them (null: the layout
     // reads the device copies back)
     const double *host_rho0 = nullptr, *host_prog = nullptr;
