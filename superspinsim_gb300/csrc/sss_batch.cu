@@ -2175,10 +2175,21 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
         // when each SM has one trajectory, and 64 a slot when it has more)
         const long n = p->auto_lanes_ntraj > 0 ? p->auto_lanes_ntraj : ntraj;
         int ctas = kPowBigMaxCtas;
-        while (ctas > 1 && n > power_big_resident(ctas)) ctas /= 2;
+        auto resident = [&](int c) {
+            int& r = p->big_resident[c];
+            if (r < 1) r = power_big_resident(c);
+            return r;
+        };
+        while (ctas > 1 && n > resident(ctas)) ctas /= 2;
         const double slots = (double)((nnz + M + 127) / 128), per_sm = std::ceil((double)n / p->num_sms);
         const double taylor = horner_terms * std::max(105.0 * slots + 500.0, 64.0 * slots * per_sm);
         const int n_chan = (int)live.size() + (Ly.pw_switch >= 0);
+        auto dearer = [&](const PowLayout& pl) {
+            return !asked && power_big_cycles(pl) * std::ceil((double)n / std::max(1, resident(pl.ctas))) > taylor;
+        };
+        // a plan remembers its last few series: they depend on the constant
+        // coefficients and the drives' largest amplitude, not on the frequencies
+        // and phases that a sweep changes
         std::vector<double> key{(double)M};
         key.insert(key.end(), row_ptr.begin(), row_ptr.end());
         key.insert(key.end(), col.begin(), col.end());
@@ -2189,6 +2200,27 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
         if (hit != p->series_memo.end()) {
             ps = hit->second;
         } else {
+            // what the series has at least rules most layouts that do not fit or do
+            // not pay out before it is made (10 to 70 ms of one core at 171 rows)
+            auto norm1 = [&](const std::vector<double>& v) {
+                std::vector<double> sum(M, 0.0);
+                for (size_t q = 0; q < col.size(); q++) sum[col[q]] += std::fabs(v[q]);
+                return *std::max_element(sum.begin(), sum.end());
+            };
+            const double A_norm = norm1(A_hi[0]), b = live.empty() ? 0.0 : rho[0] * norm1(G[0]);
+            if (!(A_norm <= 1.0 && b <= 0.25)) return no("the exponent is too large");
+            const long least = power_least_entries(M, row_ptr, col, A_hi[0], live.empty() ? nullptr : &G[0], A_norm, b);
+            for (;; ctas *= 2) {
+                if (ctas > kPowBigMaxCtas) return no("no layout fits");
+                PowLayout q;
+                q.ctas = ctas;
+                q.L = power_big_threads(ctas);
+                q.E = (int)((least + ctas * q.L - 1) / (ctas * q.L));
+                q.mono.resize(1);
+                if (power_smem(q, M, K, Q, n_chan, 1) > kPowSmem) continue;
+                if (dearer(q)) return no("the Taylor action is cheaper");
+                break;
+            }
             if (!power_series(M, row_ptr, col, A_hi, A_lo, G, rho, &ps)) return no("the exponent is too large");
             if (p->series_memo.size() >= 8) p->series_memo.clear();
             p->series_memo[key] = ps;
@@ -2200,10 +2232,8 @@ static int power_layout(sss_plan* p, int ntraj, double dt, int F, const std::vec
             ctas *= 2;
             if (ctas > kPowBigMaxCtas) return no("no layout fits");
         }
-        const int resident = power_big_resident(ctas);
-        if (resident < 1) return no("no cluster fits on the GPU");
-        if (!asked && power_big_cycles(pl) * std::ceil((double)n / resident) > taylor)
-            return no("the Taylor action is cheaper");
+        if (resident(ctas) < 1) return no("no cluster fits on the GPU");
+        if (dearer(pl)) return no("the Taylor action is cheaper");
         for (int i = 0; i < kLaneCounts; i++) p->auto_cost[i] = p->auto_chain[i] = 0.0;
         Ly.power = true;
         Ly.ps = ps;

@@ -185,9 +185,11 @@ struct sss_plan {
         std::map<int, Built> built;
     };
     std::map<std::vector<int>, LayoutMemo> layout_memo;
-    // power series of large systems by the matrices they were made from (25 ms
-    // of host time at 171 rows): pattern, constant parts, varying generators
+    // power series of large systems by the matrices they were made from: pattern,
+    // constant parts, varying generators (1.6 ms of 16 cores at 171 rows and 5 ps;
+    // new values of a laser or a drive's amplitude pay it)
     std::map<std::vector<double>, sss::PowSeries> series_memo;
+    int big_resident[sss::kPowBigMaxCtas + 1] = {};   // clusters of so many CTAs the GPU holds (0: not asked yet)
     int batch_variant = 0;  // 0: register variant when it fits, 2: shared-memory variant,
                             // 3: one-chain register variant, 4: row-part variant
     int device = 0;

@@ -25,9 +25,14 @@
 // power_pack() deals the entries to the lanes of a group.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
+#include <functional>
 #include <numeric>
+#include <system_error>
+#include <thread>
+#include <utility>
 #include <vector>
 
 namespace sss {
@@ -101,6 +106,166 @@ inline dd dd_div(dd a, double j) {
     const double r = std::fma(-q, j, a.hi) + a.lo;
     return two_sum(q, r / j);
 }
+
+// The matrices of a power series, column by column: [column][table][monomial][row].
+struct Columns {
+    int M = 0, n_live = 0, nm = 0, n_tab = 0;
+    double drop = 0.0;
+    const std::vector<std::vector<int>>* lower = nullptr;   // monomial less one factor, or -1
+    std::vector<double> size;                               // largest value of each monomial
+    // a matrix by columns, without its zeros
+    struct Sparse {
+        std::vector<int> ptr, row;
+        std::vector<dd> val;
+        Sparse(int M, const std::vector<int>& row_ptr, const std::vector<int>& col, const std::vector<double>& hi,
+               const std::vector<double>* lo)
+            : ptr(M + 1, 0) {
+            for (size_t q = 0; q < col.size(); q++) ptr[col[q] + 1] += hi[q] != 0.0;
+            std::partial_sum(ptr.begin(), ptr.end(), ptr.begin());
+            row.resize(ptr.back());
+            val.resize(ptr.back());
+            std::vector<int> at(ptr.begin(), ptr.end() - 1);
+            for (int r = 0; r < M; r++)
+                for (int q = row_ptr[r]; q < row_ptr[r + 1]; q++)
+                    if (hi[q] != 0.0) {
+                        row[at[col[q]]] = r;
+                        val[at[col[q]]++] = {hi[q], lo ? (*lo)[q] : 0.0};
+                    }
+        }
+        void add(const double* x, double* y) const {
+            for (int k = 0; k + 1 < (int)ptr.size(); k++)
+                if (x[k] != 0.0)
+                    for (int q = ptr[k]; q < ptr[k + 1]; q++) y[row[q]] += val[q].hi * x[k];
+        }
+    };
+    std::vector<Sparse> A, G;                               // constant part of each table, varying generators
+    std::vector<double> C, lo;
+    std::vector<char> keep;
+
+    // what one thread needs, allocated before it starts
+    struct Scratch {
+        std::vector<dd> D, Dn, Cd;
+        std::vector<double> T, N;                           // [monomial][row]
+        std::vector<char> alive, next;                      // monomials with terms left
+        std::vector<std::pair<double, int>> sorted;
+        Scratch(int M, int nm)
+            : D(M), Dn(M), Cd(M), T((size_t)nm * M), N((size_t)nm * M), alive(nm), next(nm), sorted((size_t)nm * M) {}
+    };
+
+    // Taylor terms T_j of column c, all monomials at once.  The constant part
+    // is in double-double until a term's rounding no longer shows in the low
+    // parts (2^-53 of it below 2^-7 of what is dropped).
+    void run(int c, Scratch& s) {
+        for (int tab = 0; tab < n_tab; tab++) {
+            double* Cc = &C[((size_t)c * n_tab + tab) * nm * M];
+            const Sparse& a = A[tab];
+            std::fill(s.D.begin(), s.D.end(), dd{0.0, 0.0});
+            std::fill(s.Cd.begin(), s.Cd.end(), dd{0.0, 0.0});
+            std::fill(s.T.begin(), s.T.end(), 0.0);
+            s.D[c] = {1.0, 0.0};
+            s.T[c] = 1.0;
+            std::fill(s.alive.begin(), s.alive.end(), 0);
+            s.alive[0] = s.next[0] = 1;
+            bool exact = true;
+            for (int j = 1; j <= 60; j++) {
+                double big = 0.0;
+                std::fill(s.N.begin(), s.N.end(), 0.0);
+                if (exact) {
+                    std::fill(s.Dn.begin(), s.Dn.end(), dd{0.0, 0.0});
+                    for (int k = 0; k < M; k++) {
+                        if (s.D[k].hi == 0.0) continue;
+                        for (int q = a.ptr[k]; q < a.ptr[k + 1]; q++)
+                            s.Dn[a.row[q]] = dd_add(s.Dn[a.row[q]], dd_mul(a.val[q], s.D[k]));
+                    }
+                    for (int r = 0; r < M; r++) {
+                        if (s.Dn[r].hi == 0.0) continue;
+                        s.Dn[r] = dd_div(s.Dn[r], j);
+                        s.Cd[r] = dd_add(s.Cd[r], s.Dn[r]);
+                        s.N[r] = s.Dn[r].hi;
+                        big = std::max(big, std::fabs(s.Dn[r].hi));
+                    }
+                    s.D.swap(s.Dn);
+                    exact = std::ldexp(big, -53) > std::ldexp(drop, -7);
+                } else {
+                    a.add(s.T.data(), s.N.data());
+                    for (int r = 0; r < M; r++) {
+                        s.N[r] /= j;
+                        s.Cd[r] = dd_add(s.Cd[r], {s.N[r], 0.0});
+                        big = std::max(big, std::fabs(s.N[r]));
+                    }
+                }
+                for (int m = 1; m < nm; m++) {
+                    double* n = &s.N[(size_t)m * M];
+                    double most = 0.0;
+                    if (s.alive[m]) a.add(&s.T[(size_t)m * M], n);
+                    bool fed = s.alive[m];
+                    for (int g = 0; g < n_live; g++)
+                        if ((*lower)[m][g] >= 0 && s.alive[(*lower)[m][g]]) {
+                            G[g].add(&s.T[(size_t)(*lower)[m][g] * M], n);
+                            fed = true;
+                        }
+                    s.next[m] = 0;
+                    if (!fed) continue;
+                    double* cm = Cc + (size_t)m * M;
+                    for (int r = 0; r < M; r++) {
+                        n[r] /= j;
+                        cm[r] += n[r];
+                        most = std::max(most, std::fabs(n[r]));
+                    }
+                    // a monomial whose terms no longer show, at its largest value,
+                    // feeds nothing any more
+                    most *= size[m];
+                    s.next[m] = most >= std::ldexp(drop, -10);
+                    big = std::max(big, most);
+                }
+                s.T.swap(s.N);
+                s.alive.swap(s.next);
+                if (big < std::ldexp(drop, -10)) break;
+            }
+            for (int r = 0; r < M; r++) {
+                Cc[r] = s.Cd[r].hi;
+                lo[((size_t)c * n_tab + tab) * M + r] = s.Cd[r].lo;
+            }
+        }
+        // all but the smallest entries (by their largest value over the tables)
+        // whose sum stays below the bound
+        int n = 0;
+        for (int m = 0; m < nm; m++)
+            for (int r = 0; r < M; r++) {
+                double v = 0.0;
+                for (int tab = 0; tab < n_tab; tab++)
+                    v = std::max(v, std::fabs(C[(((size_t)c * n_tab + tab) * nm + m) * M + r]));
+                v *= size[m];
+                if (v > 0.0) s.sorted[n++] = {v, m * M + r};
+            }
+        std::sort(s.sorted.begin(), s.sorted.begin() + n);
+        double sum = 0.0;
+        for (int i = 0; i < n; i++) {
+            sum += s.sorted[i].first;
+            if (sum > drop) keep[(size_t)c * nm * M + s.sorted[i].second] = 1;
+        }
+    }
+};
+
+// All columns, on as many threads as `work` (multiply-adds of a Taylor term) is
+// worth; a thread that cannot be started leaves its share to the others.
+inline void run_columns(Columns& w, double work) {
+    int want = (int)std::min({16.0, work / 1e5, (double)w.M});
+    if (want > 1) want = std::min(want, (int)std::thread::hardware_concurrency());   // (a system call)
+    std::vector<Columns::Scratch> scratch(std::max(1, want), Columns::Scratch(w.M, w.nm));
+    std::atomic<int> next{0};
+    auto body = [&](Columns::Scratch& s) {
+        for (int c = next++; c < w.M; c = next++) w.run(c, s);
+    };
+    std::vector<std::thread> helpers;
+    helpers.reserve(scratch.size());
+    try {
+        for (size_t i = 1; i < scratch.size(); i++) helpers.emplace_back(body, std::ref(scratch[i]));
+    } catch (const std::system_error&) {
+    }
+    body(scratch[0]);
+    for (std::thread& t : helpers) t.join();
+}
 }  // namespace pow_detail
 
 // The power series on a square pattern of M rows (CSR row_ptr/col).
@@ -165,123 +330,55 @@ inline bool power_series(int M, const std::vector<int>& row_ptr, const std::vect
             al[g]--;
             lower[m][g] = (int)(std::find(ps.mono.begin(), ps.mono.end(), al) - ps.mono.begin());
         }
-    const size_t MM = (size_t)M * M;
-    std::vector<std::vector<double>> C((size_t)n_tab * nm, std::vector<double>(MM, 0.0));
-    std::vector<std::vector<double>> C0lo(n_tab, std::vector<double>(MM, 0.0));
-    std::vector<std::vector<double>> T(nm, std::vector<double>(MM)), Nx(nm, std::vector<double>(MM));
-    std::vector<dd> D(MM), Dn(MM), Cd(MM);
-    for (int tab = 0; tab < n_tab; tab++) {
-        for (auto& t : T) std::fill(t.begin(), t.end(), 0.0);
-        std::fill(D.begin(), D.end(), dd{0.0, 0.0});
-        std::fill(Cd.begin(), Cd.end(), dd{0.0, 0.0});
-        for (int i = 0; i < M; i++) {
-            D[(size_t)i * M + i] = {1.0, 0.0};
-            T[0][(size_t)i * M + i] = 1.0;
-        }
-        std::vector<std::vector<double>*> Ct(nm);
-        for (int m = 0; m < nm; m++) Ct[m] = &C[(size_t)tab * nm + m];
-        const std::vector<double>&ah = A_hi[tab], &al = A_lo[tab];
-        for (int j = 1; j <= 60; j++) {
-            double big = 0.0;
-            for (int r = 0; r < M; r++) {
-                dd* dn = &Dn[(size_t)r * M];
-                std::fill(dn, dn + M, dd{0.0, 0.0});
-                for (int q = row_ptr[r]; q < row_ptr[r + 1]; q++) {
-                    if (ah[q] == 0.0) continue;
-                    const dd* dc = &D[(size_t)col[q] * M];
-                    const dd a{ah[q], al[q]};
-                    for (int c = 0; c < M; c++)
-                        if (dc[c].hi != 0.0) dn[c] = dd_add(dn[c], dd_mul(a, dc[c]));
-                }
-                for (int c = 0; c < M; c++) {
-                    if (dn[c].hi == 0.0) continue;
-                    dn[c] = dd_div(dn[c], j);
-                    Cd[(size_t)r * M + c] = dd_add(Cd[(size_t)r * M + c], dn[c]);
-                    big = std::max(big, std::fabs(dn[c].hi));
-                }
-            }
-            for (int m = nm - 1; m >= 1; m--) {
-                for (int r = 0; r < M; r++) {
-                    double* n = &Nx[m][(size_t)r * M];
-                    std::fill(n, n + M, 0.0);
-                    for (int q = row_ptr[r]; q < row_ptr[r + 1]; q++) {
-                        if (ah[q] != 0.0) {
-                            const double a = ah[q], *t = &T[m][(size_t)col[q] * M];
-                            for (int c = 0; c < M; c++) n[c] += a * t[c];
-                        }
-                        for (int g = 0; g < n_live; g++) {
-                            if (lower[m][g] < 0 || G[g][q] == 0.0) continue;
-                            const double a = G[g][q], *t = &T[lower[m][g]][(size_t)col[q] * M];
-                            for (int c = 0; c < M; c++) n[c] += a * t[c];
-                        }
-                    }
-                    double* cm = &(*Ct[m])[(size_t)r * M];
-                    for (int c = 0; c < M; c++) {
-                        n[c] /= j;
-                        cm[c] += n[c];
-                        big = std::max(big, std::fabs(n[c]));
-                    }
-                }
-            }
-            D.swap(Dn);
-            for (size_t i = 0; i < MM; i++) T[0][i] = D[i].hi;
-            for (int m = 1; m < nm; m++) T[m].swap(Nx[m]);
-            if (big < 1e-26) break;
-        }
-        for (size_t i = 0; i < MM; i++) {
-            (*Ct[0])[i] = Cd[i].hi;
-            C0lo[tab][i] = Cd[i].lo;
-        }
-    }
-    // keep, per column, all but the smallest entries (by their largest value
-    // over the tables) whose sum stays below the bound
-    std::vector<char> keep((size_t)nm * MM, 0);
-    std::vector<std::pair<double, size_t>> colv;
-    std::vector<double> size(nm, 1.0);   // largest value of each monomial
+    // the columns of all matrices are independent: dealt to a few threads where
+    // there is work for them
+    pow_detail::Columns w;
+    w.M = M;
+    w.n_live = n_live;
+    w.nm = nm;
+    w.n_tab = n_tab;
+    w.drop = drop;
+    w.lower = &lower;
+    for (int tab = 0; tab < n_tab; tab++) w.A.emplace_back(M, row_ptr, col, A_hi[tab], &A_lo[tab]);
+    for (int g = 0; g < n_live; g++) w.G.emplace_back(M, row_ptr, col, G[g], nullptr);
+    w.size.assign(nm, 1.0);
     for (int m = 0; m < nm; m++)
-        for (int g = 0; g < n_live; g++) size[m] *= std::pow(rho[g], ps.mono[m][g]);
-    for (int c = 0; c < M; c++) {
-        colv.clear();
+        for (int g = 0; g < n_live; g++) w.size[m] *= std::pow(rho[g], ps.mono[m][g]);
+    w.C.assign((size_t)M * n_tab * nm * M, 0.0);
+    w.lo.assign((size_t)M * n_tab * M, 0.0);
+    w.keep.assign((size_t)M * nm * M, 0);
+    pow_detail::run_columns(w, (double)M * nnz * nm * n_tab);
+    // entries by row, then monomial, then column; a low part before its entry
+    std::vector<size_t> at((size_t)M * nm + 1, 0);
+    auto keeps_low = [&](int c, int r) {
+        double v = 0.0;
+        for (int tab = 0; tab < n_tab; tab++) v = std::max(v, std::fabs(w.lo[((size_t)c * n_tab + tab) * M + r]));
+        return v > drop;
+    };
+    for (int c = 0; c < M; c++)
+        for (int m = 0; m < nm; m++)
+            for (int r = 0; r < M; r++)
+                at[(size_t)r * nm + m + 1] += w.keep[((size_t)c * nm + m) * M + r] + (m == 0 && keeps_low(c, r));
+    std::partial_sum(at.begin(), at.end(), at.begin());
+    const size_t ne = at.back();
+    ps.ent.resize(ne);
+    ps.val.resize(ne * n_tab);
+    for (int c = 0; c < M; c++)
         for (int m = 0; m < nm; m++)
             for (int r = 0; r < M; r++) {
-                double v = 0.0;
-                for (int tab = 0; tab < n_tab; tab++)
-                    v = std::max(v, std::fabs(C[(size_t)tab * nm + m][(size_t)r * M + c]));
-                v *= size[m];
-                if (v > 0.0) colv.push_back({v, (size_t)m * MM + (size_t)r * M + c});
-            }
-        std::sort(colv.begin(), colv.end());
-        double s = 0.0;
-        for (const auto& e : colv) {
-            s += e.first;
-            if (s > drop) keep[e.second] = 1;
-        }
-    }
-    ps.ent.clear();
-    std::vector<std::pair<size_t, bool>> src;   // matrix entry, low part
-    for (int r = 0; r < M; r++)
-        for (int m = 0; m < nm; m++)
-            for (int c = 0; c < M; c++) {
-                const size_t i = (size_t)r * M + c;
-                if (m == 0) {
-                    double lo = 0.0;
-                    for (int tab = 0; tab < n_tab; tab++) lo = std::max(lo, std::fabs(C0lo[tab][i]));
-                    if (lo > drop) {
-                        ps.ent.push_back({r, c, 0});
-                        src.push_back({i, true});
-                    }
+                size_t& k = at[(size_t)r * nm + m];
+                if (m == 0 && keeps_low(c, r)) {
+                    ps.ent[k] = {r, c, 0};
+                    for (int tab = 0; tab < n_tab; tab++) ps.val[tab * ne + k] = w.lo[((size_t)c * n_tab + tab) * M + r];
+                    k++;
                 }
-                if (keep[(size_t)m * MM + i]) {
-                    ps.ent.push_back({r, c, m});
-                    src.push_back({i, false});
+                if (w.keep[((size_t)c * nm + m) * M + r]) {
+                    ps.ent[k] = {r, c, m};
+                    for (int tab = 0; tab < n_tab; tab++)
+                        ps.val[tab * ne + k] = w.C[(((size_t)c * n_tab + tab) * nm + m) * M + r];
+                    k++;
                 }
             }
-    const size_t ne = ps.ent.size();
-    ps.val.assign(ne * n_tab, 0.0);
-    for (int tab = 0; tab < n_tab; tab++)
-        for (size_t k = 0; k < ne; k++)
-            ps.val[tab * ne + k] = src[k].second ? C0lo[tab][src[k].first]
-                                                 : C[(size_t)tab * nm + ps.ent[k].mono][src[k].first];
     return true;
 }
 
@@ -612,6 +709,46 @@ inline bool power_pack_big(const PowSeries& ps, int ctas, int threads, PowLayout
 // that the reduction and the barrier stay short (21 levels, 2,000 exponentials:
 // clusters of 4 take 5.8 ms at 256 lanes and 6.9 at 512).
 inline int power_big_threads(int ctas) { return ctas == 1 ? 1024 : ctas <= 2 ? 512 : 256; }
+
+// Entries that the series of a large system has at least: the patterns of its
+// Taylor terms up to third order, each counted while its bound (norms A_norm of
+// the constant part and b of the varying one) is well above what is dropped.
+// 0.42 to 0.83 of the entries for the 21-level NV (field on and off its axis, 5
+// to 30 ps); 0.1 ms at 171 rows where the series takes 2 to 7 ms of all cores.
+inline long power_least_entries(int M, const std::vector<int>& row_ptr, const std::vector<int>& col,
+                                const std::vector<double>& A, const std::vector<double>* G, double A_norm,
+                                double b) {
+    const int words = (M + 63) / 64;
+    using Bits = std::vector<uint64_t>;
+    const double drop = std::min(kPowDrop, kPowDropSmall * std::pow(A_norm + b, 1.5));
+    auto multiply = [&](const std::vector<double>& X, const Bits& Y, Bits* out) {
+        for (int r = 0; r < M; r++)
+            for (int q = row_ptr[r]; q < row_ptr[r + 1]; q++)
+                if (X[q] != 0.0)
+                    for (int w = 0; w < words; w++) (*out)[(size_t)r * words + w] |= Y[(size_t)col[q] * words + w];
+    };
+    // P[i][k]: the terms with i factors of the constant part and k of the varying one
+    Bits P[4][4];
+    P[0][0].assign((size_t)M * words, 0);
+    for (int r = 0; r < M; r++) P[0][0][(size_t)r * words + r / 64] |= (uint64_t)1 << (r % 64);
+    long n = 0;
+    for (int k = 0; k <= (G ? 3 : 0); k++) {
+        Bits all((size_t)M * words, 0);
+        for (int i = 0; i + k <= 3; i++) {
+            if (i + k == 0) continue;
+            P[i][k].assign((size_t)M * words, 0);
+            double bound = 1.0;
+            for (int j = 1; j <= i; j++) bound *= A_norm / j;
+            for (int j = 1; j <= k; j++) bound *= b / j;
+            if (bound < 1024.0 * drop) continue;
+            if (i) multiply(A, P[i - 1][k], &P[i][k]);
+            if (k) multiply(*G, P[i][k - 1], &P[i][k]);
+            for (size_t w = 0; w < all.size(); w++) all[w] |= P[i][k][w];
+        }
+        for (uint64_t w : all) n += __builtin_popcountll(w);
+    }
+    return n;
+}
 
 // Cycles of one exponential of a cluster (one CTA per SM): issue of the busiest
 // sub-partition, reduction, and the rest as measured (operand loads of 32 warps
