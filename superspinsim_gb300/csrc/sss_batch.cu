@@ -2642,11 +2642,22 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
         Ly.pw_value[1] = vals[1];
     }
 
-    // ---- samples over which nothing varies: one map per set of values (a plan
-    // that fixes its Taylor degree steps them at that degree like the others) ----
-    if (!p->adj_forward && p->d.taylor_degree == 0 && !table && !rot && allow_register && !force_parts && !p->cols_samples && M <= kConstMaxRows &&
-        F * p->d.K >= kConstMinExps)
+    // ---- samples over which nothing varies: one map per set of values, for the
+    // kernels that know them (a plan that fixes its Taylor degree steps them at
+    // that degree like the others); the later phases of a batch take its first
+    // one's ----
+    auto constants = [&]() {
+        if (p->adj_forward || p->d.taylor_degree > 0 || table || rot || !allow_register || force_parts ||
+            p->cols_samples || M > kConstMaxRows || F * p->d.K < kConstMinExps || !(Ly.power || Ly.slots))
+            return;
+        if (p->phase_constants) {
+            Ly.cs_chan = p->phase_constants->cs_chan;
+            Ly.cs = p->phase_constants->cs;
+            Ly.cs_map = p->phase_constants->cs_map;
+            return;
+        }
         constant_layout(p, Ly, h_prog, ntraj, nch, nseg, dt, F);
+    };
 
     // ---- power-series variant: automatic where it issues fewer FP64
     // instructions than the Taylor action could, or asked for (8) ----
@@ -2657,6 +2668,7 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
         if (rc == SSS_OK) {
             Ly.nnz = nnz;
             Ly.substeps = 1;
+            constants();
             return SSS_OK;
         }
         if (power_asked || p->adj_forward) return rc;
@@ -2771,9 +2783,6 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
             t.chan_const = Ly.chan_const;
             t.chan_value = Ly.chan_value;
             t.slot_chan = Ly.slot_chan;
-            t.cs_chan = Ly.cs_chan;
-            t.cs = Ly.cs;
-            t.cs_map = Ly.cs_map;
             Ly = t;
             p->last_bank_before = known->second.bank_before;
             p->last_bank_after = known->second.bank_after;
@@ -2792,6 +2801,7 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
             Ly.nnz = nnz;
             Ly.degree = degree;
             Ly.substeps = substeps;
+            constants();
         }
         if (rc == SSS_OK || row_kernels || force_parts || rot || table) return rc;
     }
@@ -3196,6 +3206,12 @@ int batch_prepare(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nse
         std::sort(p->batch_longest.begin(), p->batch_longest.end(), std::greater<int>());
     }
     int t = 0;
+    // the first phase's constant samples are the others' too
+    struct Constants {
+        sss_plan* p;
+        BatchLayout first;
+        ~Constants() { p->phase_constants = nullptr; }
+    } constants{p, {}};
     for (int k = 0; k < kMaxPhases; k++) {
         BatchLayout Ly;
         p->auto_lanes_ntraj = phased ? std::max(1, running_after(p, t)) : 0;
@@ -3208,6 +3224,12 @@ int batch_prepare(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nse
             break;
         }
         if (k > 0 && Ly.L <= p->batch_phase[k - 1].L) break;  // no wider layout: phase k-1 runs on
+        if (phased && k == 0 && (Ly.power || Ly.slots)) {
+            constants.first.cs_chan = Ly.cs_chan;
+            constants.first.cs = Ly.cs;
+            constants.first.cs_map = Ly.cs_map;
+            p->phase_constants = &constants.first;
+        }
         BatchArgs a{};
         size_t smem = 0;
         if (int rc2 = make_args(p, Ly, ntraj, nch, nseg, dt, F, h_rw, {}, p->batch_tables[k], &a,

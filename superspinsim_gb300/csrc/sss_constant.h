@@ -114,47 +114,54 @@ struct ConstSet {
 // The sets of values that the live channels of a batch's programs
 // [b][channel][segment][5] hold together for at least dt, longest total first,
 // at most kConstMax.  A run's start and end are not known here: before the
-// first segment end and after the last one counts as long.
+// first segment end and after the last one counts as long.  One walk over the
+// channels' segments: a channel's segment lasts from the largest end before it
+// to its own, if that is larger.
 inline std::vector<ConstSet> constant_sets(const double* prog, int ntraj, int nch, int nseg,
                                            const std::vector<int>& live, double dt) {
     std::vector<ConstSet> sets;
-    std::vector<double> cut;
+    struct Channel {
+        const double* seg;      // its segments
+        int s;                  // the current one (nseg: past the last)
+        double end;
+    };
+    std::vector<Channel> at(live.size());
+    std::vector<double> v(live.size());
+    auto next = [nseg](Channel& c) {
+        const double from = c.end;
+        do c.s++;
+        while (c.s < nseg && !(c.seg[c.s * 5] > from));
+        c.end = c.s < nseg ? c.seg[c.s * 5] : INFINITY;
+    };
     for (int b = 0; b < ntraj; b++) {
-        cut.clear();
-        for (int ch : live)
-            for (int s = 0; s < nseg && ch < nch; s++) {
-                const double t = prog[(((size_t)b * nch + ch) * nseg + s) * 5];
-                if (std::isfinite(t)) cut.push_back(t);
+        for (size_t i = 0; i < live.size(); i++) {
+            at[i] = {prog + ((size_t)b * nch + live[i]) * nseg * 5, -1, -INFINITY};
+            if (live[i] < nch)
+                next(at[i]);
+            else
+                at[i] = {nullptr, nseg, INFINITY};
+        }
+        double from = -INFINITY;
+        while (true) {
+            double to = INFINITY;
+            for (const Channel& c : at) to = std::min(to, c.end);
+            const double length = std::isfinite(from) && std::isfinite(to) ? to - from : 1e3 * dt;
+            bool constant = length >= dt;
+            for (size_t i = 0; i < at.size() && constant; i++) {
+                const double* sg = at[i].s < nseg ? at[i].seg + (size_t)at[i].s * 5 : nullptr;
+                constant = !sg || (sg[2] == 0.0 && std::isfinite(sg[1]));
+                v[i] = sg ? sg[1] : 0.0;
             }
-        std::sort(cut.begin(), cut.end());
-        for (size_t i = 0; i <= cut.size(); i++) {
-            const bool first = i == 0, last = i == cut.size();
-            const double from = first ? 0.0 : cut[i - 1], to = last ? 0.0 : cut[i];
-            const double length = first || last ? 1e3 * dt : to - from;
-            if (!(length >= dt)) continue;
-            const double at = first ? (last ? 0.0 : to - 0.5 * dt) : (last ? from + 0.5 * dt : 0.5 * (from + to));
-            std::vector<double> v;
-            for (int ch : live) {
-                double x = 0.0;
-                bool constant = true;
-                for (int s = 0; s < nseg && ch < nch; s++) {
-                    const double* sg = prog + (((size_t)b * nch + ch) * nseg + s) * 5;
-                    if (!(at < sg[0])) continue;
-                    constant = sg[2] == 0.0 && std::isfinite(sg[1]);
-                    x = sg[1];
-                    break;
-                }
-                if (!constant) break;
-                v.push_back(x);
+            if (constant) {
+                size_t k = 0;
+                while (k < sets.size() && sets[k].value != v) k++;
+                if (k == sets.size() && k < 64) sets.push_back({v, 0.0});
+                if (k < sets.size()) sets[k].total += length;
             }
-            if (v.size() != live.size()) continue;
-            size_t k = 0;
-            while (k < sets.size() && sets[k].value != v) k++;
-            if (k == sets.size()) {
-                if (sets.size() >= 64) continue;
-                sets.push_back({v, 0.0});
-            }
-            sets[k].total += length;
+            if (!(to < INFINITY)) break;
+            for (Channel& c : at)
+                if (c.end == to) next(c);
+            from = to;
         }
     }
     std::stable_sort(sets.begin(), sets.end(), [](const ConstSet& a, const ConstSet& b) { return a.total > b.total; });

@@ -213,6 +213,8 @@ struct sss_plan {
     // exponential's state is stored, and a channel of two values throughout the
     // programs (they cannot change before the launch) selects a table
     bool adj_forward = false;
+    // constant samples of the batch being prepared, found for its first phase
+    const sss::BatchLayout* phase_constants = nullptr;
     int launch_active = 0;       // trajectories with work in the next launch (0: the batch)
     // prepared batch (sss_batch_prepare -> sss_batch_launch): one kernel
     // layout per phase -- a single phase, or with uneven lengths and
