@@ -2005,7 +2005,10 @@ static void constant_layout(sss_plan* p, BatchLayout& Ly, const double* h_prog, 
         row_ptr.push_back((int)col.size());
     }
     using pow_detail::dd;
-    for (const ConstSet& set : constant_sets(h_prog, ntraj, nch, nseg, Ly.cs_chan, dt)) {
+    double share = 0.0;
+    const std::vector<ConstSet> sets = constant_sets(h_prog, ntraj, nch, nseg, Ly.cs_chan, dt, &share);
+    if (nseg > kConstLong && Ly.L < 32 && share < kConstShare) return;
+    for (const ConstSet& set : sets) {
         std::vector<std::vector<dd>> ex(K);
         for (int e = 0; e < K; e++) {
             ex[e].assign(col.size(), dd{0.0, 0.0});

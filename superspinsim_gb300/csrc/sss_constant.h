@@ -21,6 +21,16 @@ namespace sss {
 constexpr int kConstMax = 8;       // sets of values of a batch
 constexpr int kConstMaxRows = 32;  // reachable rows (the products cost M^3 on the host)
 constexpr int kConstMinExps = 16;  // exponentials per sample a dense product is worth
+// Groups that share a warp stop refilling their coefficient rings together once
+// one of them skips a sample, and each refill looks every node up in the
+// program.  Programs of more segments than this take maps on such groups only
+// where constant samples make up this share of them: 4,096 programs of 128
+// segments and almost none constant, groups of 8 lanes, 320 ms with maps and 269
+// without; 1,024 of 1,000 segments at 16 lanes 443 and 358; at 32 lanes (a warp
+// to itself, 200 segments) 65.1 and 66.0; 7 segments, half of them constant, 16
+// lanes 23.6 and 23.4.
+constexpr int kConstLong = 32;
+constexpr double kConstShare = 0.3;
 
 namespace pow_detail {
 
@@ -116,10 +126,13 @@ struct ConstSet {
 // at most kConstMax.  A run's start and end are not known here: before the
 // first segment end and after the last one counts as long.  One walk over the
 // channels' segments: a channel's segment lasts from the largest end before it
-// to its own, if that is larger.
+// to its own, if that is larger.  share: the part of the programs, from time 0
+// to their last end, that whole samples inside constant stretches make up (a
+// stretch holds its length less one sample of them, wherever it starts).
 inline std::vector<ConstSet> constant_sets(const double* prog, int ntraj, int nch, int nseg,
-                                           const std::vector<int>& live, double dt) {
+                                           const std::vector<int>& live, double dt, double* share = nullptr) {
     std::vector<ConstSet> sets;
+    double held = 0.0, span = 0.0;
     struct Channel {
         const double* seg;      // its segments
         int s;                  // the current one (nseg: past the last)
@@ -157,13 +170,16 @@ inline std::vector<ConstSet> constant_sets(const double* prog, int ntraj, int nc
                 while (k < sets.size() && sets[k].value != v) k++;
                 if (k == sets.size() && k < 64) sets.push_back({v, 0.0});
                 if (k < sets.size()) sets[k].total += length;
+                if (to < INFINITY) held += std::max(0.0, to - std::max(0.0, from) - dt);
             }
             if (!(to < INFINITY)) break;
+            span += std::max(0.0, to - std::max(0.0, from));
             for (Channel& c : at)
                 if (c.end == to) next(c);
             from = to;
         }
     }
+    if (share) *share = span > 0.0 ? held / span : 0.0;
     std::stable_sort(sets.begin(), sets.end(), [](const ConstSet& a, const ConstSet& b) { return a.total > b.total; });
     if (sets.size() > (size_t)kConstMax) sets.resize(kConstMax);
     return sets;
