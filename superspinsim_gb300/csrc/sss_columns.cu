@@ -39,6 +39,7 @@ int batch_columns_launch(sss_plan* p, const BatchLayout& Ly, const BatchArgs& a,
 namespace {
 
 constexpr int kBlock = kColBlock;   // runs per block of the chain
+constexpr int kSmallSamples = 32, kSmallExps = 5;   // samples and exponentials per sample of a small call
 constexpr int kMaxTerms = 256;      // Taylor terms per exponential (dense products cost about 400)
 constexpr int kLanesPerRow = 8;     // lanes of a matrix row in the chain kernels
 
@@ -260,6 +261,13 @@ int columns_run(sss_plan* p, int ntraj, const double* h_rho0, const double* d_rh
     const int N = p->d.N;
     if (N > kPlainMaxN || p->u_n || p->d.expm != SSS_EXPM_TAYLOR || p->d.taylor_degree > 0)
         return fail(SSS_EINVAL, "not a run by columns");
+    // and the smallest calls, whose host analysis takes longer than their dense
+    // products (one trajectory, N = 4 to 9, columns against dense: F K = 1, 1 sample
+    // 98 to 132 us against 48 to 60; F K = 5, 20 samples 118 to 161 against 98 to
+    // 147; from F K = 10 on, or 40 samples in the rotating frame and 80 in the lab
+    // frame, the columns are faster)
+    if (ntraj == 1 && N <= 9 && T <= kSmallSamples && F * p->d.K <= kSmallExps)
+        return fail(SSS_EINVAL, "a call too small for columns");
     // a coefficient that is not finite is the dense path's: it reports the NaN
     // that its generator makes of every state, also of the rows it does not move
     // (1e100: the cosine's argument then stays finite)
