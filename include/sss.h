@@ -115,9 +115,11 @@ int sss_plan_set_rotating(sss_plan* plan, const double* generators_nodes,
  *   out:   ntraj*T*N  state after each of the T output samples
  * Output sample t is at t0 + dt*(t+1); each spans F fine steps of dt/F.
  * With SSS_EXPM_TAYLOR the samples' propagators are built column by column by
- * the batched kernels on the rows reachable from rho0; SSS_EXPM_REFERENCE,
- * unitary mode and exponents too large for the Taylor action build them by
- * dense products, as sss_simulate_device always does. */
+ * the batched kernels on the rows reachable from rho0.  SSS_EXPM_REFERENCE,
+ * unitary mode, a fixed Taylor degree, exponents too large for the Taylor
+ * action, programs with a coefficient that is not finite and the smallest
+ * calls (one trajectory of at most 9 entries, 32 samples and 5 exponentials per
+ * sample) build them by dense products, as sss_simulate_device always does. */
 int sss_simulate(sss_plan* plan, int ntraj, const double* rho0, int nch,
                  int nseg, const double* programs, const double* coeff_table,
                  double t0, double dt, int T, int F, double* out,
@@ -165,7 +167,8 @@ int sss_batch_run(sss_plan* plan, int ntraj, const double* rho0, int nch,
  *          sss_simulate's table with T = T_max: row (r*T_max + t)*Q + k
  *          holds the G coefficients (lab [c_L0, c_1, ...], rotating
  *          [c_1, ...]) at node k of fine step r of output sample t.
- * Runs on the row-part kernel (variant 0 or 4).  A column that holds one
+ * Runs on the row-part, slot-packed, phased or power-series kernel (variant 0,
+ * 4, 6, 7 or 8).  A column that holds one
  * value everywhere is folded into the constant part of Omega; the Taylor
  * degree follows the table's largest |coefficient| per column.  NaN or
  * infinity anywhere in the table is SSS_ENONFINITE.  The other arguments
@@ -200,7 +203,7 @@ int sss_batch_prepare(sss_plan* plan, int ntraj, const double* rho0, int nch,
  * ntraj) holds each trajectory's output-sample count, and every
  * sss_batch_launch of the prepared batch must pass the same counts (as a
  * device array).  Trajectories are then handed out longest first and,
- * with automatic lanes (variant 0 or 4), the batch is also laid out for
+ * with automatic lanes (variant 0 or 4 to 8), the batch is also laid out for
  * the wider lane groups that the trajectories still running call for as
  * the shorter ones finish: a launch switches layout at the output samples
  * where the running count stops filling the GPU, and cuts its grid to the
@@ -233,8 +236,9 @@ int sss_batch_check(sss_plan* plan, void* cuda_stream);
  * memory bound of sss_plan_set_adjoint_memory) and the backward sweep walks
  * them back; when the states of one trajectory do not fit, a checkpointed
  * sweep (about sqrt(T*F) checkpoints, each interval recomputed) runs
- * instead.  The exponential's derivative is exact for the truncated series
- * the forward pass uses.  Lab frame.  readout_weights (N) and time_weights
+ * instead.  The exponential's derivative is exact for the truncated Taylor
+ * series of the backward pass; a forward pass on the power series agrees with
+ * that series to rounding.  Lab frame.  readout_weights (N) and time_weights
  * (T) are host arrays; the rest follow `host` as in sss_batch_run. */
 int sss_adjoint_run(sss_plan* plan, int ntraj, const double* rho0, int nch,
                     int nseg, const double* programs, double t0, double dt,
@@ -315,8 +319,10 @@ int sss_plan_last_launches(const sss_plan* plan);
  * multiplication by a constant sparse matrix on the powers of the varying
  * coefficients, lab frame, at most two varying coefficients that are weak
  * per step, up to 64 reachable rows, 16 to 128 lanes (above 32 a multiple
- * of 32 up to the given count); automatic where it issues fewer FP64
- * instructions than the Taylor action could).  Automatic lanes: per lane count the cheapest
+ * of 32 up to the given count), and 65 to 512 rows on a cluster of 1 to 8
+ * CTAs per trajectory (one varying coefficient, automatic lanes and CTA
+ * size); automatic where it issues fewer FP64 instructions than the Taylor
+ * action could).  Automatic lanes: per lane count the cheapest
  * layout (FP64 instructions per Horner term), and the lane count whose
  * busiest SM sub-partition issues the fewest of them.  Configured lanes
  * also set the adjoint's forward and backward groups; for sss_adjoint_run

@@ -2704,8 +2704,8 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
         return fail(SSS_EINVAL, "the rotating frame runs on the row-part, slot-packed or phased "
                                 "kernel (variant 0, 4, 6 or 7)");
     if (table && !force_parts && p->batch_variant != 0 && !row_kernels)
-        return fail(SSS_EINVAL, "a coefficient table runs on the row-part, slot-packed or phased "
-                                "kernel (variant 0, 4, 6 or 7)");
+        return fail(SSS_EINVAL, "a coefficient table runs on the row-part, slot-packed, phased "
+                                "or power-series kernel (variant 0, 4, 6, 7 or 8)");
     if (force_parts || (allow_register && (rot || table || row_kernels || p->batch_variant == 0))) {
         const int threads_cfg = p->batch_threads > 0 ? p->batch_threads : 32;
         std::vector<char> varies(G, 0);

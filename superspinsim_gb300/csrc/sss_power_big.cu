@@ -5,15 +5,16 @@
 // The 21-level NV's series at 5 ps has 18,800 entries on 171 rows, too many
 // for one CTA's registers.  The rows are dealt to the C CTAs of a cluster; a
 // CTA keeps its coefficients and operand offsets in shared memory (10 bytes an
-// entry: 188 KB for C = 1) beside the state's copies scaled by each monomial.
+// entry: 215 KB for C = 1) beside the state's copies scaled by each monomial.
 // Per exponential every row's lanes sum their entries, reduce by shuffles, add
 // to the row and write its copies, which the CTA's warps carry into every other
 // CTA's shared memory (two alternating buffers), then one cluster barrier.
 //
-// What bounds it: FP64 issue for C = 1 (8 warps per SM sub-partition x 20
-// slots x 64 cycles), and from C = 4 on the exchange as well.  The Taylor action of the same trajectory on
-// one CTA is 9 terms with a chain of 13 to 16 slots and two barriers each,
-// 19,900 cycles per exponential at 128 lanes whatever the batch leaves idle.
+// What bounds it: FP64 issue for C = 1 (8 warps per SM sub-partition x 21
+// slots x 64 cycles), and from C = 4 on the exchange as well.  The Taylor action
+// of the same trajectory on one CTA is 9 terms with a chain of 13 to 16 slots and
+// two barriers each, 19,900 cycles per exponential at 128 lanes whatever the
+// batch leaves idle.
 #include <cooperative_groups.h>
 
 #include "sss_power.cuh"

@@ -1,4 +1,4 @@
-// Power-series kernels for groups of 32 lanes, 16, 18, 20, 22, 24, 28 slots.
+// Power-series kernels for groups of 32 lanes, 16 to 20, 22, 24 and 28 slots.
 #include "sss_power.cuh"
 
 namespace sss {
