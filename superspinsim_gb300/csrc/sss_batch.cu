@@ -2763,10 +2763,10 @@ int build_layout(sss_plan* p, int ntraj, const double* d_rho0, int nch, int nseg
         // lanes as configured, or the automatic count (auto_lanes); the search
         // is remembered in the plan (at most kLayoutMemos patterns)
         int rc = SSS_EINVAL, chosen = 0;
-        if (p->layout_memo.size() >= (size_t)kLayoutMemos) p->layout_memo.clear();
-        sss_plan::LayoutMemo& memo = p->layout_memo[layout_key(
-            Ly.row_ents, active, rows_reached, varies,
-            {threads_cfg, parts_ok, slots_ok, phased_ok, p->cols_samples > 0})];
+        const std::vector<int> key = layout_key(Ly.row_ents, active, rows_reached, varies,
+                                                {threads_cfg, parts_ok, slots_ok, phased_ok, p->cols_samples > 0});
+        if (p->layout_memo.size() >= (size_t)kLayoutMemos && !p->layout_memo.count(key)) p->layout_memo.clear();
+        sss_plan::LayoutMemo& memo = p->layout_memo[key];
         if (p->batch_lanes > 0) {
             chosen = L;
         } else {
